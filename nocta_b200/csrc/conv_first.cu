@@ -41,6 +41,7 @@ __device__ __forceinline__ void load_patch(float (&x)[K], const float* __restric
 // y (N,Ho,Wo,Cout) channels-last; weights (Cout, 27)
 __global__ void __launch_bounds__(256) fwd_kernel(float* __restrict__ y, const float* __restrict__ in, const float* __restrict__ w,
                                                   const float* __restrict__ bias, Geo g, int pixels) {
+    ncc::pdl_wait();
     extern __shared__ float ws[];  // [K][Cout] then bias [Cout]
     float* bs = ws + K * g.Cout;
     for (int i = threadIdx.x; i < K * g.Cout; i += blockDim.x) {
@@ -96,6 +97,7 @@ template <int COUT, bool STAT>
 __global__ void __launch_bounds__(256, 4) fwd_tile_kernel(float* __restrict__ y, const float* __restrict__ in,
                                                        const float* __restrict__ w, const float* __restrict__ bias, Geo g,
                                                        int tiles_h, int tiles_w, int ntiles, double* __restrict__ stat) {
+    ncc::pdl_wait();
     using T = TileGeo<COUT>;
     constexpr int CG = T::CG, TR = T::TR, ROWS = TR + 2;
     __shared__ __align__(16) float ws[K * COUT];
@@ -229,9 +231,9 @@ static int launch_fwd_tile(float* y, const float* x, const float* w, const float
     // a BatchNorm that follows can take the per-channel sums from here instead of reading y again (one slab per CTA)
     double* stat = ncc::conv_stats_wanted() ? ncc::conv_stats_buffer((size_t)grid, COUT, st) : nullptr;
     if (stat) {
-        fwd_tile_kernel<COUT, true><<<grid, 256, 0, st>>>(y, x, w, bias, g, tiles_h, tiles_w, (int)ntiles, stat);
+        ncc::launch(fwd_tile_kernel<COUT, true>, grid, 256, 0, st, y, x, w, bias, g, tiles_h, tiles_w, (int)ntiles, stat);
     } else {
-        fwd_tile_kernel<COUT, false><<<grid, 256, 0, st>>>(y, x, w, bias, g, tiles_h, tiles_w, (int)ntiles, nullptr);
+        ncc::launch(fwd_tile_kernel<COUT, false>, grid, 256, 0, st, y, x, w, bias, g, tiles_h, tiles_w, (int)ntiles, nullptr);
     }
     *stat_out = stat;
     return grid;
@@ -247,6 +249,7 @@ static int launch_fwd_tile(float* y, const float* x, const float* w, const float
 template <int COUT>
 __global__ void __launch_bounds__(256) dw_tile_kernel(float* __restrict__ partial, const float* __restrict__ dy,
                                                       const float* __restrict__ in, Geo g, int tiles_h, int tiles_w, int ntiles) {
+    ncc::pdl_wait();
     constexpr int CPT = COUT / 32, TR = 4, ROWS = TR + 2, RS = (K * CPT) | 1;
     __shared__ __align__(16) float tile[3][ROWS][TWP];
     __shared__ float red[32][RS];
@@ -329,6 +332,7 @@ __global__ void __launch_bounds__(256) dw_tile_kernel(float* __restrict__ partia
 }
 
 __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, const float* __restrict__ partial, int blocks, int Cout) {
+    ncc::pdl_wait();
     // one warp per weight: lanes stride over the per-CTA partials, fixed-order shuffle tree
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= Cout * K) return;
@@ -388,6 +392,7 @@ __global__ void __launch_bounds__(544, 1) fwd_kernel(float* __restrict__ y, cons
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    ncc::pdl_wait();   // the barriers are set up while the preceding kernel ends
     // weights = the A operand: row co, K index (ci, kh, kw) as the reference stores them, padded with zeros to 32, rounded to
     // TF32; rows 64..127 are zero (the MMA wants M = 128, those accumulator lanes are never read)
     for (int i = threadIdx.x; i < 128 * 8; i += blockDim.x) {
@@ -532,7 +537,7 @@ static int forward_tc(float* y, const float* x, const float* w, const float* bia
     const int sms = ncc::sm_count();
     const int grid = ntiles < sms ? ntiles : sms;
     double* stat = ncc::conv_stats_wanted() ? ncc::conv_stats_buffer((size_t)grid, tcf::COUT, st) : nullptr;
-    tcf::fwd_kernel<<<grid, 544, tcf::SMEM, st>>>(y, x, w, bias, g, pixels, ntiles, stat, ncc::device_error_word());
+    ncc::launch(tcf::fwd_kernel, grid, 544, tcf::SMEM, st, y, x, w, bias, g, pixels, ntiles, stat, ncc::device_error_word());
     NCC_COUNT_LAUNCH();
     const int rc = ncc::launch_status("conv_first forward (tensor core)");
     if (rc == NC_CUDA_OK && stat) ncc::conv_stats_publish(y, tcf::COUT, (long long)pixels, grid, stat);
@@ -589,6 +594,7 @@ __global__ void __launch_bounds__(320, 1) dw_kernel(const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    ncc::pdl_wait();   // barriers and tensor memory are set up while the preceding kernel ends
     // tile pairs of this CTA: local index i is pair blockIdx.x + i * gridDim.x, stage i % 2
     const int nloc = ((int)blockIdx.x < npairs) ? (npairs - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
@@ -705,9 +711,9 @@ static int weight_grad_tc(float* dW, const float* dy, const float* x, const Geo&
     if (!tc::make_map(&tm, dy, 2, dims, str, box, true)) return NC_CUDA_ERR_UNSUPPORTED;
     float* partial = (float*)ncc::scratch(2, sizeof(float) * (size_t)(2 * grid) * tcw::COUT * KP, st);
     if (!partial) return NC_CUDA_ERR_RUNTIME;
-    tcw::dw_kernel<<<grid, 320, tcw::SMEM, st>>>(tm, partial, x, g, pixels, npairs, ncc::device_error_word());
+    ncc::launch(tcw::dw_kernel, grid, 320, tcw::SMEM, st, tm, partial, x, g, pixels, npairs, ncc::device_error_word());
     NCC_COUNT_LAUNCH();
-    dw_reduce_kernel<<<ncc::ceil_div(tcw::COUT * K * 32, 256), 256, 0, st>>>(dW, partial, 2 * grid, tcw::COUT);
+    ncc::launch(dw_reduce_kernel, ncc::ceil_div(tcw::COUT * K * 32, 256), 256, 0, st, dW, partial, 2 * grid, tcw::COUT);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("conv_first weight_grad (tensor core)");
 }
@@ -748,7 +754,7 @@ int forward(float* y, const float* x, const long long xs[4], const float* w, con
     const long long cap = (long long)ncc::sm_count() * 8;
     const int grid = (int)(need < cap ? need : cap);
     const size_t smem = sizeof(float) * (size_t)(K + 1) * Cout;
-    fwd_kernel<<<grid, 256, smem, st>>>(y, x, w, bias, g, pixels);
+    ncc::launch(fwd_kernel, grid, 256, smem, st, y, x, w, bias, g, pixels);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("conv_first forward");
 }
@@ -770,10 +776,10 @@ int weight_grad(float* dW, const float* dy, const float* x, const long long xs[4
     if (blocks > ntiles) blocks = ntiles;
     float* partial = (float*)ncc::scratch(2, sizeof(float) * (size_t)blocks * Cout * KP, st);
     if (!partial) return NC_CUDA_ERR_RUNTIME;
-    if (Cout == 64) dw_tile_kernel<64><<<(int)blocks, 256, 0, st>>>(partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
-    else dw_tile_kernel<32><<<(int)blocks, 256, 0, st>>>(partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
+    if (Cout == 64) ncc::launch(dw_tile_kernel<64>, (int)blocks, 256, 0, st, partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
+    else ncc::launch(dw_tile_kernel<32>, (int)blocks, 256, 0, st, partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
     NCC_COUNT_LAUNCH();
-    dw_reduce_kernel<<<ncc::ceil_div(Cout * K * 32, 256), 256, 0, st>>>(dW, partial, (int)blocks, Cout);
+    ncc::launch(dw_reduce_kernel, ncc::ceil_div(Cout * K * 32, 256), 256, 0, st, dW, partial, (int)blocks, Cout);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("conv_first weight_grad");
 }

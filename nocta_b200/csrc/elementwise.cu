@@ -20,6 +20,7 @@ __device__ __forceinline__ float4 rnd4(float4 v) { return make_float4(round_tf32
 template <int NIN, bool RND, class F>
 __global__ void __launch_bounds__(kThreads) ew_kernel(float* __restrict__ out, const float* __restrict__ a,
                                                       const float* __restrict__ b, size_t n4, size_t n, F f) {
+    ncc::pdl_wait();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     // two vectors in flight per thread per trip
@@ -63,8 +64,8 @@ int launch_ew(float* out, const float* a, const float* b, size_t n, cudaStream_t
     bool vec = aligned16(out) && (NIN < 1 || aligned16(a)) && (NIN < 2 || aligned16(b));
     size_t n4 = vec ? n / 4 : 0;
     int grid = grid_for((long long)(vec ? (n + 3) / 4 : n), kThreads, 8);
-    if (rnd) ew_kernel<NIN, true, F><<<grid, kThreads, 0, st>>>(out, a, b, n4, n, f);
-    else ew_kernel<NIN, false, F><<<grid, kThreads, 0, st>>>(out, a, b, n4, n, f);
+    if (rnd) ncc::launch(ew_kernel<NIN, true, F>, grid, kThreads, 0, st, out, a, b, n4, n, f);
+    else ncc::launch(ew_kernel<NIN, false, F>, grid, kThreads, 0, st, out, a, b, n4, n, f);
     NCC_COUNT_LAUNCH();
     return launch_status(what);
 }
@@ -107,6 +108,7 @@ struct GeluBwdF { __device__ float operator()(float dy, float x) const { return 
 // out[i] = a[i] + b[i % inner]
 __global__ void __launch_bounds__(kThreads) bias_rows_kernel(float* __restrict__ out, const float* __restrict__ a,
                                                              const float* __restrict__ b, size_t total, int inner, int rnd) {
+    ncc::pdl_wait();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         float r = a[i] + b[i % (size_t)inner];
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) bias_rows_kernel(float* __restrict__
 // One warp per row; columns strided over lanes.  Max-subtracted exponentials, f32.
 __global__ void __launch_bounds__(kThreads) softmax_rows_kernel(float* __restrict__ out, const float* __restrict__ in,
                                                                 size_t rows, size_t cols) {
+    ncc::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -137,6 +140,7 @@ struct Dims4 { size_t shape[4]; size_t stride[4]; };
 
 __global__ void __launch_bounds__(kThreads) strided_copy_kernel(float* __restrict__ dst, const float* __restrict__ src,
                                                                 Dims4 d, size_t n) {
+    ncc::pdl_wait();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         size_t r = i;
@@ -153,6 +157,7 @@ __global__ void __launch_bounds__(kThreads) strided_copy_kernel(float* __restric
 template <bool ROUND>
 __global__ void __launch_bounds__(256) transpose_kernel(float* __restrict__ dst, const float* __restrict__ src,
                                                         int R, int Cc) {
+    ncc::pdl_wait();
     __shared__ float tile[32][33];
     const size_t base = (size_t)blockIdx.z * R * Cc;
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -179,8 +184,8 @@ int transpose_batched(float* dst, const float* src, int batch, int R, int Cc, bo
     NCC_REQUIRE(batch <= 65535 && ceil_div(R, 32) <= 65535, "transpose: grid too large");
     ProfScope prof(PROF_RELAYOUT, 8.0 * (double)batch * R * Cc, st);
     dim3 grid(ceil_div(Cc, 32), ceil_div(R, 32), batch);
-    if (round) transpose_kernel<true><<<grid, 256, 0, st>>>(dst, src, R, Cc);
-    else transpose_kernel<false><<<grid, 256, 0, st>>>(dst, src, R, Cc);
+    if (round) ncc::launch(transpose_kernel<true>, grid, 256, 0, st, dst, src, R, Cc);
+    else ncc::launch(transpose_kernel<false>, grid, 256, 0, st, dst, src, R, Cc);
     NCC_COUNT_LAUNCH();
     return launch_status("transpose");
 }
@@ -220,7 +225,7 @@ int nc_cuda_add_broadcast_batch_f32_ex(float* out, const float* a, const float* 
     if (total == 0) return NC_CUDA_OK;
     NCC_REQUIRE(out && a && b && inner > 0, "add_broadcast: bad argument");
     ProfScope prof(PROF_ELEMENTWISE, 8.0 * (double)total, (cudaStream_t)stream);
-    bias_rows_kernel<<<grid_for((long long)total, kThreads), kThreads, 0, (cudaStream_t)stream>>>(out, a, b, total, inner, round_outputs() ? 1 : 0);
+    ncc::launch(bias_rows_kernel, grid_for((long long)total, kThreads), kThreads, 0, (cudaStream_t)stream, out, a, b, total, inner, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("add_broadcast");
 }
@@ -240,7 +245,7 @@ int nc_cuda_strided_copy_f32_ex(float* dst, const float* src, const size_t shape
         strides[0] == shape[2] * shape[3] * shape[1] && shape[0] <= 65535)
         return transpose_batched(dst, src, (int)shape[0], (int)(shape[2] * shape[3]), (int)shape[1], false,
                                  (cudaStream_t)stream);
-    strided_copy_kernel<<<grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(dst, src, d, n);
+    ncc::launch(strided_copy_kernel, grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream, dst, src, d, n);
     NCC_COUNT_LAUNCH();
     return launch_status("strided_copy");
 }
@@ -268,7 +273,7 @@ int nc_cuda_gelu_backward_f32_ex(float* gi, const float* go, const float* input,
 int nc_cuda_softmax_f32_ex(float* out, const float* in, size_t batch, size_t dim, void* stream) {
     if (batch == 0 || dim == 0) return NC_CUDA_OK;
     NCC_REQUIRE(out && in, "softmax: null pointer");
-    softmax_rows_kernel<<<grid_for((long long)batch * 32, kThreads), kThreads, 0, (cudaStream_t)stream>>>(out, in, batch, dim);
+    ncc::launch(softmax_rows_kernel, grid_for((long long)batch * 32, kThreads), kThreads, 0, (cudaStream_t)stream, out, in, batch, dim);
     NCC_COUNT_LAUNCH();
     return launch_status("softmax");
 }

@@ -42,6 +42,7 @@ struct GemmStore {  // D = alpha*acc + beta*D + bias[n]   or raw partial[z][m][n
 __global__ void __launch_bounds__(256) partial_reduce_kernel(float* __restrict__ D, long long ldd, const float* __restrict__ partial,
                                                              int splits, int M, int N, const float* __restrict__ bias,
                                                              float alpha, float beta) {
+    ncc::pdl_wait();
     const size_t total = (size_t)M * N, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         float acc = 0.f;
@@ -127,6 +128,7 @@ struct ConvDwB {
 // per-channel sum of a strided (N, C, Ho, Wo) tensor: fallback for layouts that are neither dense
 // NCHW nor dense channels-last.  One block per channel, double accumulation, fixed order.
 __global__ void __launch_bounds__(256) channel_sum_strided_kernel(float* __restrict__ out, const float* __restrict__ t, ConvGeo g) {
+    ncc::pdl_wait();
     __shared__ double sh[32];
     const int c = blockIdx.x;
     const long long per = (long long)g.Ho * g.Wo, total = per * g.N;
@@ -191,7 +193,7 @@ int simt_matmul(float* C, long long ldc, MatLoad la, bool a_kfast, MatLoad lb, b
     else rc = simt::launch<false, false>(M, N, K, splits, la, lb, ep, st, "simt_gemm");
     if (rc) return rc;
     if (splits > 1) {
-        partial_reduce_kernel<<<grid_for((long long)M * N, 256), 256, 0, st>>>(C, ldc, partial, splits, M, N, bias, alpha, beta);
+        ncc::launch(partial_reduce_kernel, grid_for((long long)M * N, 256), 256, 0, st, C, ldc, partial, splits, M, N, bias, alpha, beta);
         NCC_COUNT_LAUNCH();
         return launch_status("partial_reduce");
     }
@@ -379,7 +381,7 @@ int nc_cuda_conv2d_backward_weight_f32_ex(float* dW, float* db, const float* dy,
             rc = nc_cuda_sum_axis_f32_ex(tmp, dy, (size_t)N * Cout, (size_t)g.Ho * g.Wo, 1, st);
             if (!rc) rc = column_sums(db, tmp, (size_t)N, Cout, st);
         } else {
-            channel_sum_strided_kernel<<<Cout, 256, 0, st>>>(db, dy, g);
+            ncc::launch(channel_sum_strided_kernel, Cout, 256, 0, st, db, dy, g);
             NCC_COUNT_LAUNCH();
             rc = launch_status("conv2d_backward_bias");
         }
@@ -415,7 +417,7 @@ int nc_cuda_conv2d_backward_weight_f32_ex(float* dW, float* db, const float* dy,
         rc = simt::launch<false, false>(Cout, Ncols, Kred, splits, ConvDwA{dy, g}, ConvDwB{x, g}, ep, st, "conv2d_backward_weight(simt)");
     if (rc) return rc;
     if (splits > 1) {
-        partial_reduce_kernel<<<grid_for((long long)Cout * Ncols, 256), 256, 0, st>>>(dW, Ncols, partial, splits, Cout, Ncols, nullptr, 1.f, 0.f);
+        ncc::launch(partial_reduce_kernel, grid_for((long long)Cout * Ncols, 256), 256, 0, st, dW, Ncols, partial, splits, Cout, Ncols, nullptr, 1.f, 0.f);
         NCC_COUNT_LAUNCH();
         return launch_status("partial_reduce");
     }

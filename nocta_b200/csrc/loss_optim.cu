@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(kThreads) ce_fused_kernel(float* __restrict__ 
                                                             const int64_t* __restrict__ targets, int N, int C,
                                                             float gscale, double* __restrict__ partial,
                                                             unsigned int* __restrict__ ticket, int rnd) {
+    ncc::pdl_wait();
     __shared__ double sh[32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(kThreads) mse_fused_kernel(float* __restrict__
                                                              const float* __restrict__ t, size_t n, double gscale,
                                                              double* __restrict__ partial,
                                                              unsigned int* __restrict__ ticket, int rnd) {
+    ncc::pdl_wait();
     __shared__ double sh[32];
     __shared__ bool last;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -137,6 +139,7 @@ __device__ __forceinline__ void sgd_element(float* __restrict__ p, float* __rest
 
 __global__ void __launch_bounds__(kThreads) sgd_kernel(float* __restrict__ p, float* __restrict__ v,
                                                        float* __restrict__ g, SgdArgs a, size_t n) {
+    ncc::pdl_wait();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) sgd_element(p, v, g, a, i);
 }
@@ -164,6 +167,7 @@ __device__ __forceinline__ int multi_find(const MultiTable& t, unsigned int bloc
     return lo;
 }
 __global__ void __launch_bounds__(kThreads) sgd_multi_kernel(const __grid_constant__ MultiTable t, SgdArgs a) {
+    ncc::pdl_wait();
     const int k = multi_find(t, blockIdx.x);
     const size_t begin = (size_t)(blockIdx.x - t.first_block[k]) * kMultiChunk;
     size_t end = begin + kMultiChunk;
@@ -231,10 +235,12 @@ __device__ __forceinline__ void adam_range(float* __restrict__ p, float* __restr
 __global__ void __launch_bounds__(kThreads) adam_kernel(float* __restrict__ p, float* __restrict__ m,
                                                         float* __restrict__ v, float* __restrict__ vmax,
                                                         const float* __restrict__ g, AdamArgs a, size_t n) {
+    ncc::pdl_wait();
     adam_range(p, m, v, vmax, g, a, 0, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
 __global__ void __launch_bounds__(kThreads) adam_multi_kernel(const __grid_constant__ MultiTable t, AdamArgs a) {
+    ncc::pdl_wait();
     const int k = multi_find(t, blockIdx.x);
     const size_t begin = (size_t)(blockIdx.x - t.first_block[k]) * kMultiChunk;
     size_t end = begin + kMultiChunk;
@@ -248,6 +254,7 @@ __global__ void __launch_bounds__(kThreads) adam_multi_kernel(const __grid_const
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) sum_axis_kernel(float* __restrict__ out, const float* __restrict__ in,
                                                        size_t reduce_dim, size_t inner) {
+    ncc::pdl_wait();
     __shared__ double sh[8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const size_t o = blockIdx.y;
@@ -270,6 +277,7 @@ __global__ void __launch_bounds__(256) sum_axis_kernel(float* __restrict__ out, 
 // inner == 1: one warp per output, lanes stride over the reduced axis
 __global__ void __launch_bounds__(kThreads) sum_rows_kernel(float* __restrict__ out, const float* __restrict__ in,
                                                             size_t outer, size_t reduce_dim) {
+    ncc::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t o = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < outer; o += warps) {
@@ -283,6 +291,7 @@ __global__ void __launch_bounds__(kThreads) sum_rows_kernel(float* __restrict__ 
 // First maximum per row (strict >), int64 result (src/ops/reduction.c:473-513).
 __global__ void __launch_bounds__(kThreads) argmax_rows_kernel(int64_t* __restrict__ out, const float* __restrict__ in,
                                                                size_t rows, size_t cols) {
+    ncc::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -368,7 +377,7 @@ int nc_cuda_cross_entropy_fused_f32_ex(float* loss, float* grad, const float* lo
     LossScratch ls;
     int rc = loss_scratch(&ls, (long long)N * 32, st);
     if (rc) return rc;
-    ce_fused_kernel<<<ls.blocks, kThreads, 0, st>>>(loss, grad, logits, targets, N, C, grad_scale / (float)N,
+    ncc::launch(ce_fused_kernel, ls.blocks, kThreads, 0, st, loss, grad, logits, targets, N, C, grad_scale / (float)N,
                                                     ls.partial, ls.ticket, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("cross_entropy");
@@ -382,7 +391,7 @@ int nc_cuda_mse_fused_f32_ex(float* loss, float* gp, float* gt, const float* pre
     LossScratch ls;
     int rc = loss_scratch(&ls, (long long)n, st);
     if (rc) return rc;
-    mse_fused_kernel<<<ls.blocks, kThreads, 0, st>>>(loss, gp, gt, pred, target, n,
+    ncc::launch(mse_fused_kernel, ls.blocks, kThreads, 0, st, loss, gp, gt, pred, target, n,
                                                      2.0 * (double)grad_scale / (double)n, ls.partial, ls.ticket, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("mse");
@@ -404,7 +413,7 @@ int nc_cuda_sgd_update_f32_ex(float* param, float* velocity, float* grad, double
     float* v = (momentum != 0.0) ? velocity : nullptr;
     NCC_REQUIRE(momentum == 0.0 || v, "sgd: momentum without a velocity buffer");
     ProfScope prof(PROF_SGD, (v ? 20.0 : 12.0) * (double)n, (cudaStream_t)stream);
-    sgd_kernel<<<grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(param, v, grad, a, n);
+    ncc::launch(sgd_kernel, grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream, param, v, grad, a, n);
     NCC_COUNT_LAUNCH();
     return launch_status("sgd");
 }
@@ -416,7 +425,7 @@ int nc_cuda_adam_update_f32_ex(float* param, float* m, float* v, float* v_max, c
     NCC_REQUIRE(param && m && v && grad, "adam: null pointer");
     AdamArgs a{lr, beta1, beta2, eps, weight_decay, 1.0 / bias_corr1, 1.0 / bias_corr2, grad_scale};
     ProfScope prof(PROF_ADAM, (v_max ? 36.0 : 28.0) * (double)n, (cudaStream_t)stream);
-    adam_kernel<<<grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(param, m, v, v_max, grad, a, n);
+    ncc::launch(adam_kernel, grid_for((long long)n, kThreads), kThreads, 0, (cudaStream_t)stream, param, m, v, v_max, grad, a, n);
     NCC_COUNT_LAUNCH();
     return launch_status("adam");
 }
@@ -434,7 +443,7 @@ int nc_cuda_sgd_update_multi_f32_ex(int count, float* const* params, float* cons
     for (int i = 0; i < count; i++) total += (double)numel[i];
     ProfScope prof(PROF_SGD, (momentum != 0.0 ? 20.0 : 12.0) * total, st);
     return multi_launch(count, params, momentum != 0.0 ? velocities : nullptr, nullptr, nullptr, grads, numel, "sgd_multi",
-                        [&](const MultiTable& t, unsigned int blocks) { sgd_multi_kernel<<<blocks, kThreads, 0, st>>>(t, a); });
+                        [&](const MultiTable& t, unsigned int blocks) { ncc::launch(sgd_multi_kernel, blocks, kThreads, 0, st, t, a); });
 }
 
 int nc_cuda_adam_update_multi_f32_ex(int count, float* const* params, float* const* m, float* const* v, float* const* v_max,
@@ -451,7 +460,7 @@ int nc_cuda_adam_update_multi_f32_ex(int count, float* const* params, float* con
     for (int i = 0; i < count; i++) { total += (double)numel[i]; amsgrad = amsgrad || (v_max && v_max[i]); }
     ProfScope prof(PROF_ADAM, (amsgrad ? 36.0 : 28.0) * total, st);
     return multi_launch(count, params, m, v, v_max, grads, numel, "adam_multi",
-                        [&](const MultiTable& t, unsigned int blocks) { adam_multi_kernel<<<blocks, kThreads, 0, st>>>(t, a); });
+                        [&](const MultiTable& t, unsigned int blocks) { ncc::launch(adam_multi_kernel, blocks, kThreads, 0, st, t, a); });
 }
 
 void nc_cuda_sgd_step_f32(float* param, const float* grad, float lr, size_t n) {
@@ -471,11 +480,11 @@ int nc_cuda_sum_axis_f32_ex(float* out, const float* in, size_t outer, size_t re
     cudaStream_t st = (cudaStream_t)stream;
     ProfScope prof(PROF_REDUCE, 4.0 * (double)outer * reduce_dim * inner, st);
     if (inner == 1) {
-        sum_rows_kernel<<<grid_for((long long)outer * 32, kThreads), kThreads, 0, st>>>(out, in, outer, reduce_dim);
+        ncc::launch(sum_rows_kernel, grid_for((long long)outer * 32, kThreads), kThreads, 0, st, out, in, outer, reduce_dim);
     } else {
         NCC_REQUIRE(outer <= 65535, "sum_axis: outer too large");
         dim3 grid(ceil_div((long long)inner, 32), (unsigned)outer);
-        sum_axis_kernel<<<grid, 256, 0, st>>>(out, in, reduce_dim, inner);
+        ncc::launch(sum_axis_kernel, grid, 256, 0, st, out, in, reduce_dim, inner);
     }
     NCC_COUNT_LAUNCH();
     return launch_status("sum_axis");
@@ -486,7 +495,7 @@ void nc_cuda_sum_axis_f32(float* out, const float* in, size_t outer, size_t redu
 int nc_cuda_argmax_rows_f32_ex(int64_t* out, const float* in, size_t rows, size_t cols, void* stream) {
     if (rows == 0) return NC_CUDA_OK;
     NCC_REQUIRE(out && in && cols > 0, "argmax_rows: bad argument");
-    argmax_rows_kernel<<<grid_for((long long)rows * 32, kThreads), kThreads, 0, (cudaStream_t)stream>>>(out, in, rows, cols);
+    ncc::launch(argmax_rows_kernel, grid_for((long long)rows * 32, kThreads), kThreads, 0, (cudaStream_t)stream, out, in, rows, cols);
     NCC_COUNT_LAUNCH();
     return launch_status("argmax_rows");
 }

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kThreads) ce_static_kernel(float* __restrict__
                                                              const int64_t* __restrict__ targets, int N, int C,
                                                              float gscale, double* __restrict__ partial,
                                                              unsigned int* __restrict__ ticket, int rnd) {
+    ncc::pdl_wait();
     __shared__ double sh[32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31;
@@ -126,7 +127,7 @@ extern "C" int nc_cuda_cross_entropy_fused_static_f32_ex(float* loss, float* gra
     if (blocks > kMaxBlocks) return set_status(NC_CUDA_ERR_LIMIT, "cross_entropy_static: %d CTAs exceed the fixed scratch", blocks);
     // the ticket must start at zero whatever an earlier, possibly failed, call left behind
     NCC_TRY(cudaMemsetAsync(base, 0, 16, st));
-    ce_static_kernel<<<blocks, kThreads, 0, st>>>(loss, grad, logits, targets, N, C, grad_scale / (float)N,
+    ncc::launch(ce_static_kernel, blocks, kThreads, 0, st, loss, grad, logits, targets, N, C, grad_scale / (float)N,
                                                   reinterpret_cast<double*>(base + kHeaderBytes),
                                                   reinterpret_cast<unsigned int*>(base), round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();

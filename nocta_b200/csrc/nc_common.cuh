@@ -134,6 +134,28 @@ inline int launch_status(const char* what) {
         if (!(cond)) return ncc::set_status(NC_CUDA_ERR_ARG, __VA_ARGS__);                 \
     } while (0)
 
+// Every kernel of this library is launched with programmatic stream serialisation and waits (pdl_wait) before it touches global
+// memory: the grid is set up while the one before it in the stream drains.  Measured on the 47 launches of a LeNet training step
+// 435 -> 338 us, on the 41 of the 32 x 32 conv-BatchNorm step 335 -> 265 us, VGG at batch 256 3020 -> 2920 us.
+// No kernel triggers its successor early (griddepcontrol.launch_dependents): with the trigger at the top of every kernel the
+// waiting blocks of the next grid shared the SMs with the running one, which made the long kernels 2 - 13 % slower.
+// Safe by construction: nothing is read or written ahead of the wait, and the wait is for the whole preceding grid, which
+// itself waited for the one before it.
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // the caller reads the status with launch_status()
+}
+
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Grid size for grid-stride kernels: a multiple of the SM count, capped by the work.
@@ -145,6 +167,8 @@ inline int grid_for(long long work_items, int threads, int ctas_per_sm = 8) {
 }
 
 // ---------------- device helpers ----------------
+// wait for the completion (and memory flush) of the preceding kernel of the stream: first statement of every kernel, see launch()
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

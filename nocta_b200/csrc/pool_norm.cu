@@ -25,6 +25,7 @@ template <int LAYOUT, int VEC>
 __global__ void __launch_bounds__(kThreads) maxpool_fwd_kernel(float* __restrict__ out, uint8_t* __restrict__ idx,
                                                                const float* __restrict__ in, int N, int C, int H,
                                                                int W, int Ho, int Wo, int k, int stride) {
+    ncc::pdl_wait();
     const size_t total = (size_t)N * (C / VEC) * Ho * Wo;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
@@ -76,6 +77,7 @@ template <int LAYOUT, int VEC>
 __global__ void __launch_bounds__(kThreads) maxpool_bwd_own_kernel(float* __restrict__ gin, const float* __restrict__ gout,
                                                                    const uint8_t* __restrict__ idx, int N, int C, int H,
                                                                    int W, int Ho, int Wo, int k, int stride) {
+    ncc::pdl_wait();
     const size_t total = (size_t)N * (C / VEC) * Ho * Wo;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
@@ -123,6 +125,7 @@ template <int LAYOUT>
 __global__ void __launch_bounds__(kThreads) maxpool_bwd_gather_kernel(float* __restrict__ gin, const float* __restrict__ gout,
                                                                       const uint8_t* __restrict__ idx, int N, int C, int H,
                                                                       int W, int Ho, int Wo, int k, int stride) {
+    ncc::pdl_wait();
     const size_t total = (size_t)N * C * H * W;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
@@ -158,8 +161,8 @@ int maxpool_fwd(float* out, uint8_t* idx, const float* in, int N, int C, int H, 
     const size_t total = (size_t)N * C * Ho * Wo / (vec ? 4 : 1);
     if (total == 0) return NC_CUDA_OK;
     int grid = grid_for((long long)total, kThreads);
-    if (vec) maxpool_fwd_kernel<1, 4><<<grid, kThreads, 0, st>>>(out, idx, in, N, C, H, W, Ho, Wo, k, s);
-    else maxpool_fwd_kernel<LAYOUT, 1><<<grid, kThreads, 0, st>>>(out, idx, in, N, C, H, W, Ho, Wo, k, s);
+    if (vec) ncc::launch(maxpool_fwd_kernel<1, 4>, grid, kThreads, 0, st, out, idx, in, N, C, H, W, Ho, Wo, k, s);
+    else ncc::launch(maxpool_fwd_kernel<LAYOUT, 1>, grid, kThreads, 0, st, out, idx, in, N, C, H, W, Ho, Wo, k, s);
     NCC_COUNT_LAUNCH();
     return launch_status("maxpool_forward");
 }
@@ -170,7 +173,7 @@ int maxpool_bwd(float* gin, const float* gout, const uint8_t* idx, int N, int C,
     const int Ho = (H - k) / s + 1, Wo = (W - k) / s + 1;
     if ((size_t)N * C * H * W == 0) return NC_CUDA_OK;
     if (s < k) {
-        maxpool_bwd_gather_kernel<LAYOUT><<<grid_for((long long)N * C * H * W, kThreads), kThreads, 0, st>>>(
+        ncc::launch(maxpool_bwd_gather_kernel<LAYOUT>, grid_for((long long)N * C * H * W, kThreads), kThreads, 0, st, 
             gin, gout, idx, N, C, H, W, Ho, Wo, k, s);
         NCC_COUNT_LAUNCH();
         return launch_status("maxpool_backward(gather)");
@@ -182,8 +185,8 @@ int maxpool_bwd(float* gin, const float* gout, const uint8_t* idx, int N, int C,
     const size_t total = (size_t)N * C * Ho * Wo / (vec ? 4 : 1);
     if (total == 0) return NC_CUDA_OK;
     int grid = grid_for((long long)total, kThreads);
-    if (vec) maxpool_bwd_own_kernel<1, 4><<<grid, kThreads, 0, st>>>(gin, gout, idx, N, C, H, W, Ho, Wo, k, s);
-    else maxpool_bwd_own_kernel<LAYOUT, 1><<<grid, kThreads, 0, st>>>(gin, gout, idx, N, C, H, W, Ho, Wo, k, s);
+    if (vec) ncc::launch(maxpool_bwd_own_kernel<1, 4>, grid, kThreads, 0, st, gin, gout, idx, N, C, H, W, Ho, Wo, k, s);
+    else ncc::launch(maxpool_bwd_own_kernel<LAYOUT, 1>, grid, kThreads, 0, st, gin, gout, idx, N, C, H, W, Ho, Wo, k, s);
     NCC_COUNT_LAUNCH();
     return launch_status("maxpool_backward");
 }
@@ -198,6 +201,7 @@ int maxpool_bwd(float* gin, const float* gout, const uint8_t* idx, int N, int C,
 template <class F>
 __global__ void __launch_bounds__(256) colreduce_kernel(double* __restrict__ partial, size_t rows, int cols,
                                                         size_t rows_per_slab, F f) {
+    ncc::pdl_wait();
     __shared__ double sh[2][8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + tx;
@@ -232,6 +236,7 @@ __global__ void __launch_bounds__(256) colreduce_kernel(double* __restrict__ par
 template <class F>
 __global__ void __launch_bounds__(256) colreduce4_kernel(double* __restrict__ partial, size_t rows, int cols, size_t rows_per_slab,
                                                          int TX, F f) {
+    ncc::pdl_wait();
     __shared__ double sh[256][9];
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX, TY = 256 / TX;
     const int c = (blockIdx.x * TX + tx) * 4;
@@ -281,6 +286,7 @@ __global__ void __launch_bounds__(256) colreduce4_kernel(double* __restrict__ pa
 // of `spatial` floats.
 template <class F>
 __global__ void __launch_bounds__(256) chanreduce_nchw_kernel(double* __restrict__ partial, int N, int C, int spatial, F f) {
+    ncc::pdl_wait();
     __shared__ double sh[32];
     const int c = blockIdx.x, j = blockIdx.y, J = gridDim.y;
     double a = 0.0, b = 0.0;
@@ -429,8 +435,8 @@ int launch_colreduce(double** partial_out, int* slabs_out, size_t rows, int cols
     if (slabs > 65535) { slabs = 65535; rps = (rows + slabs - 1) / slabs; slabs = (int)((rows + rps - 1) / rps); }
     double* partial = (double*)scratch(7, sizeof(double) * 2 * (size_t)slabs * cols, st);
     if (!partial) return NC_CUDA_ERR_RUNTIME;
-    if (vec) colreduce4_kernel<<<dim3(col_tiles, slabs), 256, 0, st>>>(partial, rows, cols, rps, TX, f);
-    else colreduce_kernel<<<dim3(col_tiles, slabs), 256, 0, st>>>(partial, rows, cols, rps, f);
+    if (vec) ncc::launch(colreduce4_kernel<F>, dim3(col_tiles, slabs), 256, 0, st, partial, rows, cols, rps, TX, f);
+    else ncc::launch(colreduce_kernel<F>, dim3(col_tiles, slabs), 256, 0, st, partial, rows, cols, rps, f);
     NCC_COUNT_LAUNCH();
     *partial_out = partial;
     *slabs_out = slabs;
@@ -478,6 +484,7 @@ inline int fin_grid(int C) { return (C + kFinCols - 1) / kFinCols; }
 __global__ void __launch_bounds__(kFinCols * kFinLanes) bn_fwd_finalize_kernel(const double* __restrict__ partial, int slabs, int C, double M,
                                        float* __restrict__ save_mean, float* __restrict__ save_var,
                                        float* __restrict__ run_mean, float* __restrict__ run_var, double momentum) {
+    ncc::pdl_wait();
     int c;
     double s1, s2;
     if (!combine_slabs(partial, slabs, C, &c, &s1, &s2)) return;
@@ -497,6 +504,7 @@ __global__ void __launch_bounds__(kFinCols * kFinLanes) bn_fwd_finalize_kernel(c
 // eval mode: statistics come from the running buffers (or 0 / 1 when absent)
 __global__ void bn_eval_stats_kernel(int C, float* __restrict__ save_mean, float* __restrict__ save_var,
                                      const float* __restrict__ run_mean, const float* __restrict__ run_var) {
+    ncc::pdl_wait();
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     save_mean[c] = run_mean ? run_mean[c] : 0.f;
@@ -510,6 +518,7 @@ __global__ void __launch_bounds__(kThreads) bn_apply_kernel(float* __restrict__ 
                                                             const float* __restrict__ gamma, const float* __restrict__ beta,
                                                             const float* __restrict__ mean, const float* __restrict__ var,
                                                             float eps, int C, int spatial, size_t nvec, int relu, int rnd) {
+    ncc::pdl_wait();
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += gstride) {
         const size_t e = i * VEC;
@@ -542,6 +551,7 @@ __global__ void __launch_bounds__(kThreads) bn_apply_nhwc4_kernel(float4* __rest
                                                                   const float* __restrict__ gamma, const float* __restrict__ beta,
                                                                   const float* __restrict__ mean, const float* __restrict__ var,
                                                                   float eps, int C, size_t nvec, int rnd) {
+    ncc::pdl_wait();
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x, total = gridDim.x * kThreads;
     const int c = (int)((tid * 4ull) % (unsigned)C);
     float mu[4], is[4], g[4], b[4];
@@ -575,6 +585,7 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_nhwc4_kernel(float4* __
                                                                       const float* __restrict__ mean, const float* __restrict__ var,
                                                                       const float* __restrict__ sums, float eps, float Mf, int C,
                                                                       size_t nvec, int rnd) {
+    ncc::pdl_wait();
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x, total = gridDim.x * kThreads;
     const int c = (int)((tid * 4ull) % (unsigned)C);
     float mu[4], is[4], g[4], b[4], coeff[4], s1[4], s2[4];
@@ -621,6 +632,7 @@ __global__ void __launch_bounds__(kThreads) bn_relu_pool2_fwd_kernel(float4* __r
                                                                      const float* __restrict__ beta, const float* __restrict__ mean,
                                                                      const float* __restrict__ var, float eps, int C, int H, int W,
                                                                      size_t nvec_out, int rnd) {
+    ncc::pdl_wait();
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x, total = gridDim.x * kThreads;
     const int C4 = C >> 2, Ho = H >> 1, Wo = W >> 1;
     const int c = (int)((tid * 4ull) % (unsigned)C);
@@ -705,6 +717,7 @@ __global__ void __launch_bounds__(kThreads) bn_relu_pool2_bwd_apply_kernel(float
                                                                            const float* __restrict__ mean, const float* __restrict__ var,
                                                                            const float* __restrict__ sums, float eps, float Mf, int C, int H,
                                                                            int W, size_t nvec_out, int rnd) {
+    ncc::pdl_wait();
     const unsigned tid = blockIdx.x * kThreads + threadIdx.x, total = gridDim.x * kThreads;
     const int C4 = C >> 2, Ho = H >> 1, Wo = W >> 1;
     const int c = (int)((tid * 4ull) % (unsigned)C);
@@ -759,6 +772,7 @@ inline int nhwc4_grid(size_t nvec, int C) {
 
 __global__ void __launch_bounds__(kFinCols * kFinLanes) bn_bwd_finalize_kernel(const double* __restrict__ partial, int slabs, int C,
                                        float* __restrict__ dgamma, float* __restrict__ dbeta, float* __restrict__ sums) {
+    ncc::pdl_wait();
     int c;
     double s1, s2;
     if (!combine_slabs(partial, slabs, C, &c, &s1, &s2)) return;
@@ -775,6 +789,7 @@ __global__ void __launch_bounds__(kThreads) bn_bwd_apply_kernel(float* __restric
                                                                 const float* __restrict__ gamma, const float* __restrict__ mean,
                                                                 const float* __restrict__ var, const float* __restrict__ sums,
                                                                 float eps, float Mf, int C, int spatial, size_t nvec, int rnd) {
+    ncc::pdl_wait();
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += gstride) {
         const size_t e = i * VEC;
@@ -817,7 +832,7 @@ int channel_reduce(double** partial_out, int* slabs_out, int N, int C, int spati
         if (J > 65535) J = 65535;
         double* partial = (double*)scratch(7, sizeof(double) * 2 * (size_t)J * C, st);
         if (!partial) return NC_CUDA_ERR_RUNTIME;
-        chanreduce_nchw_kernel<<<dim3(C, J), 256, 0, st>>>(partial, N, C, spatial, fflat);
+        ncc::launch(chanreduce_nchw_kernel<FF>, dim3(C, J), 256, 0, st, partial, N, C, spatial, fflat);
         NCC_COUNT_LAUNCH();
         *partial_out = partial;
         *slabs_out = J;
@@ -831,6 +846,7 @@ int channel_reduce(double** partial_out, int* slabs_out, int N, int C, int spati
 __global__ void __launch_bounds__(kThreads) ln_fwd_kernel(float* __restrict__ y, const float* __restrict__ x,
                                                           const float* __restrict__ gamma, const float* __restrict__ beta,
                                                           size_t rows, int cols, float eps, int rnd) {
+    ncc::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -857,6 +873,7 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_rows_kernel(float* __restrict
                                                                const float* __restrict__ dy, const float* __restrict__ x,
                                                                const float* __restrict__ gamma, size_t rows, int cols,
                                                                float eps, int rnd) {
+    ncc::pdl_wait();
     const int lane = threadIdx.x & 31;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
     for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -892,6 +909,7 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_rows_kernel(float* __restrict
 
 __global__ void __launch_bounds__(kFinCols * kFinLanes) ln_param_finalize_kernel(const double* __restrict__ partial, int slabs, int cols,
                                          float* __restrict__ dgamma, float* __restrict__ dbeta) {
+    ncc::pdl_wait();
     int c;
     double s1, s2;
     if (!combine_slabs(partial, slabs, cols, &c, &s1, &s2)) return;
@@ -921,7 +939,7 @@ int ncc::column_sums(float* out, const float* in, size_t rows, int cols, cudaStr
     int slabs = 0;
     int rc = launch_colreduce(&partial, &slabs, rows, cols, al16(in), ColSum{in, cols}, st);
     if (rc) return rc;
-    ln_param_finalize_kernel<<<fin_grid(cols), kFinCols * kFinLanes, 0, st>>>(partial, slabs, cols, out, nullptr);
+    ncc::launch(ln_param_finalize_kernel, fin_grid(cols), kFinCols * kFinLanes, 0, st, partial, slabs, cols, out, nullptr);
     NCC_COUNT_LAUNCH();
     return launch_status("column_sums");
 }
@@ -983,10 +1001,10 @@ int nc_cuda_batchnorm_forward_f32_ex(float* y, const float* x, const float* gamm
             int rc = channel_reduce(&partial, &slabs, N, C, spatial, layout, BnFwdSum{x, C}, BnFwdSumFlat{x}, al16(x), st);
             if (rc) return rc;
         }
-        bn_fwd_finalize_kernel<<<fin_grid(C), kFinCols * kFinLanes, 0, st>>>(partial, slabs, C, (double)N * spatial, save_mean,
+        ncc::launch(bn_fwd_finalize_kernel, fin_grid(C), kFinCols * kFinLanes, 0, st, partial, slabs, C, (double)N * spatial, save_mean,
                                                                 save_var, run_mean, run_var, momentum);
     } else {
-        bn_eval_stats_kernel<<<ceil_div(C, 128), 128, 0, st>>>(C, save_mean, save_var, run_mean, run_var);
+        ncc::launch(bn_eval_stats_kernel, ceil_div(C, 128), 128, 0, st, C, save_mean, save_var, run_mean, run_var);
     }
     NCC_COUNT_LAUNCH();
     const bool al = ((uintptr_t)y % 16 == 0) && ((uintptr_t)x % 16 == 0);
@@ -995,15 +1013,15 @@ int nc_cuda_batchnorm_forward_f32_ex(float* y, const float* x, const float* gamm
     const int grid = grid_for((long long)nvec, kThreads);
     const float fe = (float)eps;
     if (layout == 0) {
-        if (vec) bn_apply_kernel<0, 4><<<grid, kThreads, 0, st>>>(y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
-        else bn_apply_kernel<0, 1><<<grid, kThreads, 0, st>>>(y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
+        if (vec) ncc::launch(bn_apply_kernel<0, 4>, grid, kThreads, 0, st, y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
+        else ncc::launch(bn_apply_kernel<0, 1>, grid, kThreads, 0, st, y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
     } else {
         if (vec) {
             const int g4 = nhwc4_grid(nvec, C);
             const int flags = (round_outputs() ? 1 : 0) | (total * 4 > kStreamBytes ? 2 : 0);
-            if (relu) bn_apply_nhwc4_kernel<1><<<g4, kThreads, 0, st>>>((float4*)y, (const float4*)x, gamma, beta, save_mean, save_var, fe, C, nvec, flags);
-            else bn_apply_nhwc4_kernel<0><<<g4, kThreads, 0, st>>>((float4*)y, (const float4*)x, gamma, beta, save_mean, save_var, fe, C, nvec, flags);
-        } else bn_apply_kernel<1, 1><<<grid, kThreads, 0, st>>>(y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
+            if (relu) ncc::launch(bn_apply_nhwc4_kernel<1>, g4, kThreads, 0, st, (float4*)y, (const float4*)x, gamma, beta, save_mean, save_var, fe, C, nvec, flags);
+            else ncc::launch(bn_apply_nhwc4_kernel<0>, g4, kThreads, 0, st, (float4*)y, (const float4*)x, gamma, beta, save_mean, save_var, fe, C, nvec, flags);
+        } else ncc::launch(bn_apply_kernel<1, 1>, grid, kThreads, 0, st, y, x, gamma, beta, save_mean, save_var, fe, C, spatial, nvec, relu, round_outputs() ? 1 : 0);
     }
     NCC_COUNT_LAUNCH();
     return launch_status("batchnorm_forward");
@@ -1034,7 +1052,7 @@ int nc_cuda_batchnorm_backward_f32_ex(float* dx, float* dgamma, float* dbeta, co
     }
     float* sums = (float*)scratch(6, sizeof(float) * 2 * (size_t)C, st);
     if (!sums) return NC_CUDA_ERR_RUNTIME;
-    bn_bwd_finalize_kernel<<<fin_grid(C), kFinCols * kFinLanes, 0, st>>>(partial, slabs, C, dgamma, dbeta, sums);
+    ncc::launch(bn_bwd_finalize_kernel, fin_grid(C), kFinCols * kFinLanes, 0, st, partial, slabs, C, dgamma, dbeta, sums);
     NCC_COUNT_LAUNCH();
     const bool al = ((uintptr_t)dx % 16 == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0) &&
                     (!relu_out || (uintptr_t)relu_out % 16 == 0);
@@ -1043,16 +1061,16 @@ int nc_cuda_batchnorm_backward_f32_ex(float* dx, float* dgamma, float* dbeta, co
     const int grid = grid_for((long long)nvec, kThreads);
     const float Mf = (float)((double)N * spatial);
     if (layout == 0) {
-        if (vec) bn_bwd_apply_kernel<0, 4><<<grid, kThreads, 0, st>>>(dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
-        else bn_bwd_apply_kernel<0, 1><<<grid, kThreads, 0, st>>>(dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
+        if (vec) ncc::launch(bn_bwd_apply_kernel<0, 4>, grid, kThreads, 0, st, dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
+        else ncc::launch(bn_bwd_apply_kernel<0, 1>, grid, kThreads, 0, st, dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
     } else {
         if (vec) {
             const int g4 = nhwc4_grid(nvec, C);
             const int rnd = (round_outputs() ? 1 : 0) | (total * 4 > kStreamBytes ? 2 : 0);
-            if (relu_out) bn_bwd_apply_nhwc4_kernel<1><<<g4, kThreads, 0, st>>>((float4*)dx, (const float4*)dy, (const float4*)x, (const float4*)relu_out, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
-            else if (relu_recompute) bn_bwd_apply_nhwc4_kernel<2><<<g4, kThreads, 0, st>>>((float4*)dx, (const float4*)dy, (const float4*)x, nullptr, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
-            else bn_bwd_apply_nhwc4_kernel<0><<<g4, kThreads, 0, st>>>((float4*)dx, (const float4*)dy, (const float4*)x, nullptr, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
-        } else bn_bwd_apply_kernel<1, 1><<<grid, kThreads, 0, st>>>(dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
+            if (relu_out) ncc::launch(bn_bwd_apply_nhwc4_kernel<1>, g4, kThreads, 0, st, (float4*)dx, (const float4*)dy, (const float4*)x, (const float4*)relu_out, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
+            else if (relu_recompute) ncc::launch(bn_bwd_apply_nhwc4_kernel<2>, g4, kThreads, 0, st, (float4*)dx, (const float4*)dy, (const float4*)x, nullptr, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
+            else ncc::launch(bn_bwd_apply_nhwc4_kernel<0>, g4, kThreads, 0, st, (float4*)dx, (const float4*)dy, (const float4*)x, nullptr, gamma, relu_beta, save_mean, save_var, sums, fe, Mf, C, nvec, rnd);
+        } else ncc::launch(bn_bwd_apply_kernel<1, 1>, grid, kThreads, 0, st, dx, dy, x, mask, gamma, save_mean, save_var, sums, fe, Mf, C, spatial, nvec, round_outputs() ? 1 : 0);
     }
     NCC_COUNT_LAUNCH();
     return launch_status("batchnorm_backward");
@@ -1077,14 +1095,14 @@ int nc_cuda_batchnorm_relu_maxpool2_forward_f32_ex(float* pooled, uint8_t* argma
             int rc = channel_reduce(&partial, &slabs, N, C, H * W, 1, BnFwdSum{x, C}, BnFwdSumFlat{x}, true, st);
             if (rc) return rc;
         }
-        bn_fwd_finalize_kernel<<<fin_grid(C), kFinCols * kFinLanes, 0, st>>>(partial, slabs, C, (double)N * H * W, save_mean, save_var, run_mean,
+        ncc::launch(bn_fwd_finalize_kernel, fin_grid(C), kFinCols * kFinLanes, 0, st, partial, slabs, C, (double)N * H * W, save_mean, save_var, run_mean,
                                                                 run_var, momentum);
     } else {
-        bn_eval_stats_kernel<<<ceil_div(C, 128), 128, 0, st>>>(C, save_mean, save_var, run_mean, run_var);
+        ncc::launch(bn_eval_stats_kernel, ceil_div(C, 128), 128, 0, st, C, save_mean, save_var, run_mean, run_var);
     }
     NCC_COUNT_LAUNCH();
     const size_t nvec = (size_t)N * (H / 2) * (W / 2) * (C / 4);
-    bn_relu_pool2_fwd_kernel<<<nhwc4_grid(nvec, C), kThreads, 0, st>>>((float4*)pooled, (uchar4*)argmax, (const float4*)x, gamma, beta,
+    ncc::launch(bn_relu_pool2_fwd_kernel, nhwc4_grid(nvec, C), kThreads, 0, st, (float4*)pooled, (uchar4*)argmax, (const float4*)x, gamma, beta,
                                                                      save_mean, save_var, (float)eps, C, H, W, nvec,
                                                                      round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
@@ -1111,10 +1129,10 @@ int nc_cuda_batchnorm_relu_maxpool2_backward_f32_ex(float* dx, float* dgamma, fl
     if (rc) return rc;
     float* sums = (float*)scratch(6, sizeof(float) * 2 * (size_t)C, st);
     if (!sums) return NC_CUDA_ERR_RUNTIME;
-    bn_bwd_finalize_kernel<<<fin_grid(C), kFinCols * kFinLanes, 0, st>>>(partial, slabs, C, dgamma, dbeta, sums);
+    ncc::launch(bn_bwd_finalize_kernel, fin_grid(C), kFinCols * kFinLanes, 0, st, partial, slabs, C, dgamma, dbeta, sums);
     NCC_COUNT_LAUNCH();
     const size_t nvec = prow * (C / 4);
-    bn_relu_pool2_bwd_apply_kernel<<<nhwc4_grid(nvec, C), kThreads, 0, st>>>((float4*)dx, (const float4*)dpooled, (const uchar4*)argmax,
+    ncc::launch(bn_relu_pool2_bwd_apply_kernel, nhwc4_grid(nvec, C), kThreads, 0, st, (float4*)dx, (const float4*)dpooled, (const uchar4*)argmax,
                                                                            (const float4*)x, gamma, beta, save_mean, save_var, sums, fe,
                                                                            (float)((double)N * H * W), C, H, W, nvec,
                                                                            round_outputs() ? 1 : 0);
@@ -1140,7 +1158,7 @@ int nc_cuda_layernorm_forward_f32_ex(float* y, const float* x, const float* gamm
     if (rows == 0 || cols == 0) return NC_CUDA_OK;
     NCC_REQUIRE(y && x && cols <= 0x7fffffff, "layernorm_forward: bad argument");
     ProfScope prof(PROF_LAYERNORM, 8.0 * (double)rows * cols, (cudaStream_t)stream);
-    ln_fwd_kernel<<<grid_for((long long)rows * 32, kThreads), kThreads, 0, (cudaStream_t)stream>>>(y, x, gamma, beta, rows, (int)cols, (float)eps, round_outputs() ? 1 : 0);
+    ncc::launch(ln_fwd_kernel, grid_for((long long)rows * 32, kThreads), kThreads, 0, (cudaStream_t)stream, y, x, gamma, beta, rows, (int)cols, (float)eps, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("layernorm_forward");
 }
@@ -1158,7 +1176,7 @@ int nc_cuda_layernorm_backward_f32_ex(float* dx, float* dgamma, float* dbeta, co
         stats = (float2*)scratch(6, sizeof(float2) * rows, st);
         if (!stats) return NC_CUDA_ERR_RUNTIME;
     }
-    ln_bwd_rows_kernel<<<grid_for((long long)rows * 32, kThreads), kThreads, 0, st>>>(dx, stats, dy, x, gamma, rows, (int)cols, (float)eps, round_outputs() ? 1 : 0);
+    ncc::launch(ln_bwd_rows_kernel, grid_for((long long)rows * 32, kThreads), kThreads, 0, st, dx, stats, dy, x, gamma, rows, (int)cols, (float)eps, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     if (params) {
         int C = (int)cols;
@@ -1166,7 +1184,7 @@ int nc_cuda_layernorm_backward_f32_ex(float* dx, float* dgamma, float* dbeta, co
         int slabs = 0;
         int rc = launch_colreduce(&partial, &slabs, rows, C, al16(dy) && al16(x), LnParamSum{dy, x, stats, C}, st);
         if (rc) return rc;
-        ln_param_finalize_kernel<<<fin_grid(C), kFinCols * kFinLanes, 0, st>>>(partial, slabs, C, dgamma, dbeta);
+        ncc::launch(ln_param_finalize_kernel, fin_grid(C), kFinCols * kFinLanes, 0, st, partial, slabs, C, dgamma, dbeta);
         NCC_COUNT_LAUNCH();
     }
     return launch_status("layernorm_backward");

@@ -16,6 +16,7 @@ constexpr int TM = 64, TN = 64, TK = 16, PADN = 4;
 // by the host so global loads coalesce along the contiguous index.
 template <bool A_KFAST, bool B_KFAST, class LA, class LB, class EP>
 __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, int k_per_split, LA la, LB lb, EP ep) {
+    ncc::pdl_wait();
     __shared__ __align__(16) float As[TK][TM + PADN];
     __shared__ __align__(16) float Bs[TK][TN + PADN];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -84,7 +85,7 @@ inline int launch(int M, int N, int K, int splits, LA la, LB lb, EP ep, cudaStre
     dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, splits);
     if (grid.y > 65535 || grid.z > 65535)
         return ncc::set_status(NC_CUDA_ERR_UNSUPPORTED, "%s: grid too large for the SIMT path", what);
-    gemm_kernel<A_KFAST, B_KFAST><<<grid, 256, 0, st>>>(M, N, K, kps, la, lb, ep);
+    ncc::launch(gemm_kernel<A_KFAST, B_KFAST, LA, LB, EP>, grid, 256, 0, st, M, N, K, kps, la, lb, ep);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status(what);
 }

@@ -151,6 +151,7 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    ncc::pdl_wait();   // barriers and tensor memory are set up while the preceding kernel ends
     volatile int* abortp = &abort_flag;
     const int total_tiles = p.tiles_px * p.tiles_m;  // t -> (pixel tile fastest, then channel tile)
     const int ntaps = p.kH * p.kW;
@@ -652,6 +653,7 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    ncc::pdl_wait();   // barriers and tensor memory are set up while the preceding kernel ends
     volatile int* abortp = &abort_flag;
     const int total_work = p.items * p.splits;   // w -> (item fastest, then split): CTAs that run together share pixels
     const int ksteps_w = p.TW >> 3;
@@ -877,7 +879,7 @@ static int convh_launch(const CUtensorMap& tw, const CUtensorMap& tx, ConvhParam
     }
     {
         ncc::ProfScope prof(ncc::prof_role(), flops, st, true);
-        convh_kernel<PXM, NCH, DUAL><<<grid, PXM ? (NCH <= 2 ? 288 : 224) : (DUAL ? 352 : 320), smem, st>>>(tw, tx, p);
+        ncc::launch(convh_kernel<PXM, NCH, DUAL>, grid, PXM ? (NCH <= 2 ? 288 : 224) : (DUAL ? 352 : 320), smem, st, tw, tx, p);
     }
     NCC_COUNT_LAUNCH();
     if (p.bnx) ncc::bn_fold_publish(p.D, (int)slabs, p.stat);
@@ -1054,8 +1056,8 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
     }
     {
         ncc::ProfScope prof(ncc::prof_role(), flops, st, true);
-        if (shift) dwh_kernel<true><<<grid, 256, smem, st>>>(tdy, tx, p);
-        else dwh_kernel<false><<<grid, 256, smem, st>>>(tdy, tx, p);
+        if (shift) ncc::launch(dwh_kernel<true>, grid, 256, smem, st, tdy, tx, p);
+        else ncc::launch(dwh_kernel<false>, grid, 256, smem, st, tdy, tx, p);
     }
     NCC_COUNT_LAUNCH();
     const int rc = ncc::launch_status("dwh_kernel");

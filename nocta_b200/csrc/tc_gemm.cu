@@ -143,6 +143,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
+    ncc::pdl_wait();   // barriers and tensor memory are set up while the preceding kernel ends
     volatile int* abortp = &abort_flag;
 
     // Persistent CTA: walks output tiles t = blockIdx.x, blockIdx.x + gridDim.x, ...
@@ -630,6 +631,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ D, long long ldd, const float* __restrict__ partial,
                                                             int splits, int M, int N, const float* __restrict__ bias,
                                                             float alpha, float beta) {
+    ncc::pdl_wait();
     const size_t total = (size_t)M * N, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         double acc = 0.0;   // the splits are combined in double, in order: no rounding that grows with their number
@@ -656,6 +658,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
 // before the first one is added, and only the single write per element is scattered.
 __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, const float* __restrict__ partial, int splits,
                                                         int Cout, int Cin, int kH, int kW) {
+    ncc::pdl_wait();
     const int T = kH * kW;
     const size_t total = (size_t)Cout * Cin * T, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t src = (size_t)blockIdx.x * blockDim.x + threadIdx.x; src < total; src += stride) {
@@ -680,6 +683,7 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, 
 template <bool DX>
 __global__ void __launch_bounds__(256) pack_weights_kernel(float* __restrict__ wp, const float* __restrict__ w, int Cout, int Cin,
                                                            int kH, int kW, int round) {
+    ncc::pdl_wait();
     const size_t total = (size_t)Cout * Cin * kH * kW, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         size_t r = i;
@@ -715,7 +719,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcPara
     }
     {
         ncc::ProfScope prof(ncc::prof_role(), p.flops, st, true);
-        kern<<<grid, ProdCfg<A_MN, B_MN, BN>::THREADS, Cfg::SMEM_BYTES, st>>>(ta, tb, p);
+        ncc::launch(kern, grid, ProdCfg<A_MN, B_MN, BN>::THREADS, Cfg::SMEM_BYTES, st, ta, tb, p);
     }
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("tc_kernel");
@@ -798,7 +802,7 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
     else rc = launch_bn<true, true>(bn, mode, ta, tb, p, grid, st);
     if (rc) return rc;
     if (splits > 1) {
-        splitk_reduce_kernel<<<ncc::grid_for((long long)M * N, 256), 256, 0, st>>>(D, ldd, p.partial, splits, M, N, bias, alpha, beta);
+        ncc::launch(splitk_reduce_kernel, ncc::grid_for((long long)M * N, 256), 256, 0, st, D, ldd, p.partial, splits, M, N, bias, alpha, beta);
         NCC_COUNT_LAUNCH();
         return ncc::launch_status("splitk_reduce");
     }
@@ -953,18 +957,18 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
 }
 
 int dw_reduce(float* dW, const float* partial, int splits, int Cout, int Cin, int kH, int kW, cudaStream_t st) {
-    dw_reduce_kernel<<<ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st>>>(dW, partial, splits, Cout, Cin, kH, kW);
+    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, dW, partial, splits, Cout, Cin, kH, kW);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("dw_reduce");
 }
 
 int pack_weights_fwd(float* wp, const float* w, int Cout, int Cin, int kH, int kW, bool round, cudaStream_t st) {
-    pack_weights_kernel<false><<<ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st>>>(wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
+    ncc::launch(pack_weights_kernel<false>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_fwd");
 }
 int pack_weights_dx(float* wp, const float* w, int Cout, int Cin, int kH, int kW, bool round, cudaStream_t st) {
-    pack_weights_kernel<true><<<ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st>>>(wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
+    ncc::launch(pack_weights_kernel<true>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_dx");
 }
