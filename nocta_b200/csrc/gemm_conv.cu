@@ -8,6 +8,8 @@
 #include "nc_common.cuh"
 #include "simt_gemm.cuh"
 #include "tc_gemm.cuh"
+#include "small_conv.cuh"
+#include "small_linear.cuh"
 #include "../../include/nocta_cuda.h"
 
 using namespace ncc;
@@ -200,16 +202,27 @@ int simt_matmul(float* C, long long ldc, MatLoad la, bool a_kfast, MatLoad lb, b
     return NC_CUDA_OK;
 }
 
+// Products that stay below the tensor-core tile sizes run on the kernels of small_linear.cu: up to 2^24 multiply-adds (there
+// the 64 x 64 tiles leave most of the chip idle: 64 rows, 256 -> 120 features 11 us against 3 us), and any product of at most
+// 32 rows against a K-major matrix, which is bound by reading that matrix.
+bool small_product(int M, int N, int K, bool rows_form) { return (long long)M * N * K < (1ll << 24) || (rows_form && M <= 32); }
+
 // C(M,N) = alpha * A' * B'^T + beta*C + bias, A' = (M,K) logical, B' = (N,K) logical.
 //   a_mn: A stored (K,M);  b_mn: B stored (K,N).
+// round_b: B is a parameter that TF32 mode reads rounded (the tensor-core path gets a rounded copy instead).
 int gemm_dispatch(float* C, int ldc, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N,
-                  int K, const float* bias, float alpha, float beta, cudaStream_t st) {
+                  int K, const float* bias, float alpha, float beta, cudaStream_t st, bool round_b = false) {
     if (M <= 0 || N <= 0) return NC_CUDA_OK;
     NCC_REQUIRE(C && (K == 0 || (A && B)), "gemm: null pointer");
     if (tc_enabled() && K > 0) {
         prof_set_role(a_mn ? (b_mn ? PROF_GEMM_TN : PROF_GEMM_TT) : (b_mn ? PROF_GEMM_NN : PROF_GEMM_NT));
         int rc = tc::gemm(C, ldc, A, lda, a_mn, B, ldb, b_mn, M, N, K, bias, alpha, beta, tc_mode(), st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
+    }
+    if (alpha == 1.f && beta == 0.f && K > 0) {
+        if (!a_mn && !b_mn && small_product(M, N, K, true)) return small_rows(C, ldc, A, lda, B, ldb, bias, M, N, K, round_b, st);
+        if (b_mn && !bias && small_product(M, N, K, false))
+            return small_columns(ColumnsJob{C, ldc, A, a_mn ? 1 : lda, a_mn ? lda : 1, B, ldb, nullptr, M, N, K, round_b}, ColumnsJob{}, st);
     }
     MatLoad la{A, a_mn ? 1 : lda, a_mn ? lda : 1};
     MatLoad lb{B, b_mn ? 1 : ldb, b_mn ? ldb : 1};
@@ -220,8 +233,8 @@ int gemm_dispatch(float* C, int ldc, const float* A, int lda, bool a_mn, const f
 // NCHW tensors can still use the tensor-core kernels: re-lay them out channels-last in library
 // scratch (one coalesced transpose pass each way).  Worth it only when the channel counts tile.
 bool relayout_ok(const ConvGeo& g) {
-    return tc_enabled() && g.stride == 1 && (g.Cin % 32 == 0) && (g.Cout % 32 == 0) && g.kH == g.kW &&
-           g.kH - 1 - g.pad >= 0 && (long long)g.N * g.Ho * g.Wo >= 128 && g.N <= 65535 &&
+    return tc_enabled() && g.stride <= 2 && tc::conv_eligible(g.Cin, g.Cout, (long long)g.N * g.Ho * g.Wo) && g.kH == g.kW &&
+           g.kH - 1 - g.pad >= 0 && g.N <= 65535 &&
            is_nchw(g.xs, g.Cin, g.H, g.W) && is_nchw(g.ys, g.Cout, g.Ho, g.Wo);
 }
 // In plain TF32 mode the relayout pass also rounds to the nearest TF32 value, so the tensor core's
@@ -235,11 +248,18 @@ void nhwc_strides(size_t s[4], int C, int H, int W) {
     s[0] = (size_t)H * W * C; s[1] = 1; s[2] = (size_t)W * C; s[3] = (size_t)C;
 }
 
-// Parameters keep their full f32 value in memory; in plain TF32 mode the Linear GEMMs read a copy
-// rounded to the nearest TF32 value (library scratch) so that the tensor core's truncation of its
-// operands is exact.  Skipped when the GEMM will run on the FP32 SIMT kernel anyway (fewer than 128 rows).
-const float* conditioned_weight(const float* W, size_t n, int rows, cudaStream_t st) {
-    if (math_mode() != NC_CUDA_MATH_TF32 || rows < 128) return W;
+bool pieces16(const void* p, int ld) { return (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// whether tc::gemm takes this product
+bool tc_takes(int M, int N, int K, const float* A, int lda, const float* B, int ldb) {
+    return tc_enabled() && tc::gemm_eligible(M, N, K, pieces16(A, lda) && pieces16(B, ldb));
+}
+// Parameters keep their full f32 value in memory; in plain TF32 mode the Linear GEMMs read them rounded to the nearest TF32 value
+// (so that the tensor core's truncation of its operands is exact): a copy in library scratch, except where the kernel that
+// takes the product rounds by itself (small products, and operands that are copied for TMA anyway).  Not below 128 rows.
+bool rounds_weight(int rows) { return math_mode() == NC_CUDA_MATH_TF32 && rows >= 128; }
+const float* conditioned_weight(const float* W, int rows, int in_f, int out_f, bool on_tc, bool small, cudaStream_t st) {
+    if (!rounds_weight(rows) || (on_tc ? !pieces16(W, in_f) : small)) return W;
+    const size_t n = (size_t)in_f * out_f;
     float* Wr = (float*)scratch(3, sizeof(float) * n, st);
     if (!Wr) return nullptr;
     if (nc_cuda_round_tf32_f32_ex(Wr, W, n, st)) return nullptr;
@@ -265,10 +285,10 @@ void nc_cuda_matmul_f32(float* C, const float* A, const float* B, int M, int N, 
 int nc_cuda_linear_forward_f32_ex(float* y, const float* x, const float* W, const float* bias, int batch, int in_f,
                                   int out_f, void* stream) {
     NCC_REQUIRE(y && x && W && batch > 0 && in_f > 0 && out_f > 0, "linear_forward: bad argument");
-    const float* Wc = conditioned_weight(W, (size_t)out_f * in_f, batch, (cudaStream_t)stream);
+    const float* Wc = conditioned_weight(W, batch, in_f, out_f, tc_takes(batch, out_f, in_f, x, in_f, W, in_f), small_product(batch, out_f, in_f, true), (cudaStream_t)stream);
     if (!Wc) return NC_CUDA_ERR_RUNTIME;
     // y(B,out) = x(B,in) * W(out,in)^T : both operands K-major
-    return gemm_dispatch(y, out_f, x, in_f, false, Wc, in_f, false, batch, out_f, in_f, bias, 1.f, 0.f, (cudaStream_t)stream);
+    return gemm_dispatch(y, out_f, x, in_f, false, Wc, in_f, false, batch, out_f, in_f, bias, 1.f, 0.f, (cudaStream_t)stream, rounds_weight(batch));
 }
 
 int nc_cuda_linear_backward_f32_ex(float* dx, float* dW, float* db, const float* dy, const float* x, const float* W,
@@ -276,12 +296,19 @@ int nc_cuda_linear_backward_f32_ex(float* dx, float* dW, float* db, const float*
     NCC_REQUIRE(dy && batch > 0 && in_f > 0 && out_f > 0, "linear_backward: bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
+    const bool dx_tc = tc_takes(batch, in_f, out_f, dy, out_f, W, in_f), dw_tc = tc_takes(out_f, in_f, batch, dy, out_f, x, in_f);
+    if (dW && x && !dw_tc && (!dx || (W && !dx_tc)) && small_product(batch, in_f, out_f, false)) {
+        // both products and the bias gradient in one launch
+        ProfScope prof(PROF_REDUCE, 4.0 * ((double)batch * (in_f + out_f) + 2.0 * (double)in_f * out_f), st);
+        return small_columns(ColumnsJob{dx, in_f, dy, out_f, 1, W, in_f, nullptr, batch, in_f, out_f, rounds_weight(batch)},
+                             ColumnsJob{dW, in_f, dy, 1, out_f, x, in_f, db, out_f, in_f, batch, 0}, st);
+    }
     if (dx) {
         NCC_REQUIRE(W, "linear_backward: dx needs W");
-        const float* Wc = conditioned_weight(W, (size_t)out_f * in_f, batch, st);
+        const float* Wc = conditioned_weight(W, batch, in_f, out_f, dx_tc, small_product(batch, in_f, out_f, false), st);
         if (!Wc) return NC_CUDA_ERR_RUNTIME;
         // dx(B,in) = dy(B,out) * W(out,in): A K-major (k = out), B stored (K = out, N = in) -> MN-major
-        rc = gemm_dispatch(dx, in_f, dy, out_f, false, Wc, in_f, true, batch, in_f, out_f, nullptr, 1.f, 0.f, st);
+        rc = gemm_dispatch(dx, in_f, dy, out_f, false, Wc, in_f, true, batch, in_f, out_f, nullptr, 1.f, 0.f, st, rounds_weight(batch));
         if (rc) return rc;
     }
     if (dW) {
@@ -318,18 +345,27 @@ int nc_cuda_conv2d_forward_f32_ex(float* y, const size_t ys[4], const float* x, 
         if (rc) return rc;
         return nc_cuda_nhwc_to_nchw_f32_ex(y, yh, N, Cout, g.Ho * g.Wo, st);
     }
-    if (tc_enabled() && stride == 1 && is_nhwc(g.xs, Cin, H, W) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
-        float* wp = (float*)scratch(3, sizeof(float) * (size_t)Cout * Cin * kH * kW, st);
+    const bool tc1 = stride == 1 && tc::conv_eligible(Cin, Cout, (long long)N * g.Ho * g.Wo);
+    const bool tc2 = tc::conv_strided_eligible(Cin, Cout, (long long)N * g.Ho * g.Wo, kH, kW, stride);
+    if (tc_enabled() && (tc1 || tc2) && is_nhwc(g.xs, Cin, H, W) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
+        const int planes = tc::mode_planes(tc_mode());
+        float* wp = (float*)scratch(3, sizeof(float) * (size_t)Cout * Cin * kH * kW * planes, st);
         if (!wp) return NC_CUDA_ERR_RUNTIME;
-        rc = tc::pack_weights_fwd(wp, w, Cout, Cin, kH, kW, round_in_relayout() != 0, st);
-        if (rc) return rc;
+        rc = tc::pack_weights_fwd(wp, w, Cout, Cin, kH, kW, planes, st);
         prof_set_role(PROF_CONV_FWD);
-        rc = tc::conv_nhwc(y, x, wp, bias, N, H, W, Cin, Cout, kH, kW, pad, tc_mode(), st);
+        if (!rc)
+            rc = tc1 ? tc::conv_nhwc(y, x, wp, bias, N, H, W, Cin, Cout, kH, kW, pad, tc_mode(), st)
+                     : tc::conv_strided_nhwc(y, x, wp, bias, N, H, W, Cin, Cout, kH, kW, stride, pad, tc_mode(), st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
     if (convfirst::eligible(Cin, kH, kW, stride, Cout) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
         ProfScope prof(PROF_CONV_FIRST, 4.0 * ((double)N * g.Ho * g.Wo * Cout + (double)N * Cin * H * W), st);
         rc = convfirst::forward(y, x, g.xs, w, bias, N, H, W, Cout, pad, st);
+        if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
+    }
+    if (stride == 1 && kH == kW) {
+        ProfScope prof(PROF_CONV_FIRST, 4.0 * ((double)N * g.Ho * g.Wo * Cout + (double)N * Cin * H * W), st);
+        rc = smallconv::conv(y, g.ys, x, g.xs, w, bias, N, Cin, H, W, Cout, kH, pad, false, st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
     const int M = N * g.Ho * g.Wo, K = Cin * kH * kW;
@@ -347,15 +383,23 @@ int nc_cuda_conv2d_backward_input_f32_ex(float* dx, const size_t xs[4], const fl
     ConvGeo g;
     int rc = make_geo(&g, ys, xs, N, Cin, H, W, Cout, kH, kW, stride, pad);
     if (rc) return rc;
-    if (tc_enabled() && stride == 1 && kH - 1 - pad >= 0 && kW == kH && is_nhwc(g.xs, Cin, H, W) &&
-        is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
-        float* wp = (float*)scratch(3, sizeof(float) * (size_t)Cout * Cin * kH * kW, st);
+    const bool tc1 = stride == 1 && kH - 1 - pad >= 0 && kW == kH && tc::conv_eligible(Cout, Cin, (long long)N * H * W);
+    const bool tc2 = tc::conv_strided_eligible(Cout, Cin, (long long)N * H * W, kH, kW, stride);
+    if (tc_enabled() && (tc1 || tc2) && is_nhwc(g.xs, Cin, H, W) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
+        const int planes = tc::mode_planes(tc_mode());
+        float* wp = (float*)scratch(3, sizeof(float) * (size_t)Cout * Cin * kH * kW * planes, st);
         if (!wp) return NC_CUDA_ERR_RUNTIME;
-        rc = tc::pack_weights_dx(wp, w, Cout, Cin, kH, kW, round_in_relayout() != 0, st);
-        if (rc) return rc;
-        // dx = conv(dy, flipped weights) with padding k-1-pad; roles of Cin and Cout swap
+        rc = tc::pack_weights_dx(wp, w, Cout, Cin, kH, kW, stride, pad, planes, st);
+        // stride 1: dx = conv(dy, reversed weights) with padding k-1-pad; roles of Cin and Cout swap
         prof_set_role(PROF_CONV_DX);
-        rc = tc::conv_nhwc(dx, dy, wp, nullptr, N, g.Ho, g.Wo, Cout, Cin, kH, kW, kH - 1 - pad, tc_mode(), st);
+        if (!rc)
+            rc = tc1 ? tc::conv_nhwc(dx, dy, wp, nullptr, N, g.Ho, g.Wo, Cout, Cin, kH, kW, kH - 1 - pad, tc_mode(), st)
+                     : tc::conv_dx_strided_nhwc(dx, dy, wp, N, H, W, Cin, Cout, kH, kW, stride, pad, tc_mode(), st);
+        if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
+    }
+    if (stride == 1 && kH == kW && kH - 1 - pad >= 0) {
+        ProfScope prof(PROF_CONV_FIRST, 4.0 * ((double)N * g.Ho * g.Wo * Cout + (double)N * Cin * H * W), st);
+        rc = smallconv::conv(dx, g.xs, dy, g.ys, w, nullptr, N, Cout, g.Ho, g.Wo, Cin, kH, kH - 1 - pad, true, st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
     const int M = N * H * W, K = Cout * kH * kW;
@@ -372,6 +416,11 @@ int nc_cuda_conv2d_backward_weight_f32_ex(float* dW, float* db, const float* dy,
     size_t dummy[4] = {0, 0, 0, 0};
     int rc = make_geo(&g, ys, xs ? xs : dummy, N, Cin, H, W, Cout, kH, kW, stride, pad);
     if (rc) return rc;
+    if (dW && stride == 1 && kH == kW && (Cin < 16 || Cout < 16) && !convfirst::eligible(Cin, kH, kW, stride, Cout)) {
+        ProfScope prof(PROF_CONV_FIRST, 4.0 * ((double)N * g.Ho * g.Wo * Cout + (double)N * Cin * H * W), st);
+        rc = smallconv::weight_grad(dW, db, dy, g.ys, x, g.xs, N, Cin, H, W, Cout, kH, pad, st);
+        if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
+    }
     if (db) {
         if (is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
             rc = column_sums(db, dy, (size_t)N * g.Ho * g.Wo, Cout, st);
@@ -388,9 +437,9 @@ int nc_cuda_conv2d_backward_weight_f32_ex(float* dW, float* db, const float* dy,
         if (rc) return rc;
     }
     if (!dW) return NC_CUDA_OK;
-    if (tc_enabled() && stride == 1 && is_nhwc(g.xs, Cin, H, W) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
+    if (tc_enabled() && is_nhwc(g.xs, Cin, H, W) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {
         prof_set_role(PROF_CONV_DW);
-        rc = tc::conv_dw_nhwc(dW, dy, x, N, H, W, Cin, Cout, kH, kW, pad, tc_mode(), st);
+        rc = tc::conv_dw_nhwc(dW, dy, x, N, H, W, Cin, Cout, kH, kW, stride, pad, tc_mode(), st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
     if (convfirst::eligible(Cin, kH, kW, stride, Cout) && is_nhwc(g.ys, Cout, g.Ho, g.Wo)) {

@@ -16,14 +16,35 @@ constexpr int kThreads = 256;
 // ---------------------------------------------------------------------------------------------
 // Cross entropy.  One warp per row: row max, sum of exponentials (f32 exp, double accumulation of
 // the per-row loss), optional gradient (softmax - onehot) * scale.  Per-block partial losses go to
-// `partial`; the last block (ticket counter) adds them in index order, so the loss is bit-stable
-// from run to run.
+// `partial`; the block that draws the last ticket adds them with a fixed assignment to threads and a
+// fixed tree, so the loss is bit-stable from run to run.
 // ---------------------------------------------------------------------------------------------
+
+// Ticket of the loss kernels: atomicInc wraps it to zero with the last block of a launch, so no launch or memset prepares it
+// (zero when the module is loaded).  As with the partial sums, loss calls of one device must not overlap.
+__device__ unsigned int g_loss_ticket;
+
+// Every block calls this with its own sum; the last one to arrive writes total / n.  One thread adding a few hundred partials
+// in a row took longer than the rest of the kernel.
+__device__ __forceinline__ void combine_loss(double own, double n, float* loss, double* partial, double* sh) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = own;
+        __threadfence();
+        last = atomicInc(&g_loss_ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (unsigned int i = threadIdx.x; i < gridDim.x; i += blockDim.x) t += __ldcg(&partial[i]);
+    t = block_sum(t, sh);
+    if (threadIdx.x == 0 && loss) *loss = (float)(t / n);
+}
 __global__ void __launch_bounds__(kThreads) ce_fused_kernel(float* __restrict__ loss, float* __restrict__ grad,
                                                             const float* __restrict__ logits,
                                                             const int64_t* __restrict__ targets, int N, int C,
-                                                            float gscale, double* __restrict__ partial,
-                                                            unsigned int* __restrict__ ticket, int rnd) {
+                                                            float gscale, double* __restrict__ partial, int rnd) {
     ncc::pdl_wait();
     __shared__ double sh[32];
     __shared__ bool last;
@@ -55,56 +76,46 @@ __global__ void __launch_bounds__(kThreads) ce_fused_kernel(float* __restrict__ 
             }
         }
     }
-    double b = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = b;
-        __threadfence();
-        unsigned int t = atomicAdd(ticket, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double tot = 0.0;
-        for (unsigned int i = 0; i < gridDim.x; i++) tot += ((volatile double*)partial)[i];
-        if (loss) *loss = (float)(tot / (double)N);
-        *ticket = 0;
-    }
+    combine_loss(block_sum(acc, sh), (double)N, loss, partial, sh);
 }
 
+// Bound by memory: 12 bytes an element with a gradient.  16.8 MB operands: 38 -> 11 us with float4 accesses and the parallel
+// combination of the partial sums.
+template <bool VEC>
 __global__ void __launch_bounds__(kThreads) mse_fused_kernel(float* __restrict__ loss, float* __restrict__ gp,
                                                              float* __restrict__ gt, const float* __restrict__ p,
                                                              const float* __restrict__ t, size_t n, double gscale,
-                                                             double* __restrict__ partial,
-                                                             unsigned int* __restrict__ ticket, int rnd) {
+                                                             double* __restrict__ partial, int rnd) {
     ncc::pdl_wait();
     __shared__ double sh[32];
-    __shared__ bool last;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     double acc = 0.0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float d = p[i] - t[i];
+    auto one = [&](float a, float b) {
+        const float d = a - b;
         acc += (double)d * (double)d;
-        float g = (float)(gscale * (double)d);
-        if (rnd) g = round_tf32(g);
-        if (gp) gp[i] = g;
-        if (gt) gt[i] = -g;
+        const float g = (float)(gscale * (double)d);
+        return rnd ? round_tf32(g) : g;
+    };
+    const size_t n4 = VEC ? n / 4 : 0;
+    auto four = [&](const float4& a, const float4& b, size_t i) {
+        const float4 g = make_float4(one(a.x, b.x), one(a.y, b.y), one(a.z, b.z), one(a.w, b.w));
+        if (gp) reinterpret_cast<float4*>(gp)[i] = g;
+        if (gt) reinterpret_cast<float4*>(gt)[i] = make_float4(-g.x, -g.y, -g.z, -g.w);
+    };
+    size_t i = first;
+    for (; i + stride < n4; i += 2 * stride) {   // two vectors of each operand in flight
+        const float4 a0 = reinterpret_cast<const float4*>(p)[i], b0 = reinterpret_cast<const float4*>(t)[i];
+        const float4 a1 = reinterpret_cast<const float4*>(p)[i + stride], b1 = reinterpret_cast<const float4*>(t)[i + stride];
+        four(a0, b0, i);
+        four(a1, b1, i + stride);
     }
-    double b = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = b;
-        __threadfence();
-        unsigned int k = atomicAdd(ticket, 1u);
-        last = (k == gridDim.x - 1);
+    for (; i < n4; i += stride) four(reinterpret_cast<const float4*>(p)[i], reinterpret_cast<const float4*>(t)[i], i);
+    for (size_t k = n4 * 4 + first; k < n; k += stride) {
+        const float g = one(p[k], t[k]);
+        if (gp) gp[k] = g;
+        if (gt) gt[k] = -g;
     }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double tot = 0.0;
-        for (unsigned int i = 0; i < gridDim.x; i++) tot += ((volatile double*)partial)[i];
-        if (loss) *loss = (float)(tot / (double)n);
-        *ticket = 0;
-    }
+    combine_loss(block_sum(acc, sh), (double)n, loss, partial, sh);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -312,23 +323,10 @@ __global__ void __launch_bounds__(kThreads) argmax_rows_kernel(int64_t* __restri
     }
 }
 
-struct LossScratch { double* partial; unsigned int* ticket; int blocks; };
-
-int loss_scratch(LossScratch* ls, long long work, cudaStream_t st) {
-    int blocks = grid_for(work, kThreads, 4);
-    // layout: [ticket (16 B)] [partials]
-    char* base = (char*)scratch(0, 16 + sizeof(double) * (size_t)blocks, st);
-    if (!base) return NC_CUDA_ERR_RUNTIME;
-    // The ticket must start at zero.  A kernel resets it when it ends, but not after a failed or aborted launch, and a
-    // regrown block starts with arbitrary contents: clear it in stream order on every call (calls on different streams
-    // share this one block and must not overlap).
-    cudaError_t e = cudaMemsetAsync(base, 0, 16, st);
-    if (e != cudaSuccess) return set_status(NC_CUDA_ERR_RUNTIME, "loss scratch memset failed");
-    ++g_epoch;
-    ls->ticket = (unsigned int*)base;
-    ls->partial = (double*)(base + 16);
-    ls->blocks = blocks;
-    return NC_CUDA_OK;
+// one partial sum per block of a loss kernel
+double* loss_scratch(long long work, int* blocks, cudaStream_t st) {
+    *blocks = grid_for(work, kThreads, 4);
+    return (double*)scratch(0, sizeof(double) * (size_t)*blocks, st);
 }
 
 // Fills launch tables of at most kMultiMax tensors from the caller's host arrays and launches `launch` for each.
@@ -374,11 +372,11 @@ int nc_cuda_cross_entropy_fused_f32_ex(float* loss, float* grad, const float* lo
     NCC_REQUIRE(logits && targets && N > 0 && C > 0, "cross_entropy: bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     ProfScope prof(PROF_LOSS, (grad ? 8.0 : 4.0) * (double)N * C + 8.0 * N, st);
-    LossScratch ls;
-    int rc = loss_scratch(&ls, (long long)N * 32, st);
-    if (rc) return rc;
-    ncc::launch(ce_fused_kernel, ls.blocks, kThreads, 0, st, loss, grad, logits, targets, N, C, grad_scale / (float)N,
-                                                    ls.partial, ls.ticket, round_outputs() ? 1 : 0);
+    int blocks = 0;
+    double* partial = loss_scratch((long long)N * 32, &blocks, st);
+    if (!partial) return NC_CUDA_ERR_RUNTIME;
+    ncc::launch(ce_fused_kernel, blocks, kThreads, 0, st, loss, grad, logits, targets, N, C, grad_scale / (float)N, partial,
+                round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("cross_entropy");
 }
@@ -388,11 +386,14 @@ int nc_cuda_mse_fused_f32_ex(float* loss, float* gp, float* gt, const float* pre
     NCC_REQUIRE(pred && target && n > 0, "mse: bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     ProfScope prof(PROF_LOSS, (8.0 + (gp ? 4.0 : 0.0) + (gt ? 4.0 : 0.0)) * (double)n, st);
-    LossScratch ls;
-    int rc = loss_scratch(&ls, (long long)n, st);
-    if (rc) return rc;
-    ncc::launch(mse_fused_kernel, ls.blocks, kThreads, 0, st, loss, gp, gt, pred, target, n,
-                                                     2.0 * (double)grad_scale / (double)n, ls.partial, ls.ticket, round_outputs() ? 1 : 0);
+    auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    const bool vec = al(pred) && al(target) && al(gp) && al(gt);
+    int blocks = 0;
+    double* partial = loss_scratch((long long)(vec ? (n + 3) / 4 : n), &blocks, st);
+    if (!partial) return NC_CUDA_ERR_RUNTIME;
+    const double gs = 2.0 * (double)grad_scale / (double)n;
+    if (vec) ncc::launch(mse_fused_kernel<true>, blocks, kThreads, 0, st, loss, gp, gt, pred, target, n, gs, partial, round_outputs() ? 1 : 0);
+    else ncc::launch(mse_fused_kernel<false>, blocks, kThreads, 0, st, loss, gp, gt, pred, target, n, gs, partial, round_outputs() ? 1 : 0);
     NCC_COUNT_LAUNCH();
     return launch_status("mse");
 }

@@ -142,18 +142,24 @@ inline int launch_status(const char* what) {
 // Safe by construction: nothing is read or written ahead of the wait, and the wait is for the whole preceding grid, which
 // itself waited for the one before it.
 template <class... P, class... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_clusters(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = {cluster, 1, 1};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // the caller reads the status with launch_status()
+}
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    launch_clusters(1, kernel, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
@@ -195,6 +201,20 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     double r = (lane < nw) ? sh[lane] : 0.0;
     r = warp_sum(r);
     return r;
+}
+
+// Thread-block clusters: rank of this block, barrier over the cluster, and a float of another block's shared memory (`local` is
+// the address of the same variable in this block).
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(const float* local, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(local), r;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
 }
 
 // Round an f32 to the nearest TF32 value (ties away), keeping it in an f32 container.

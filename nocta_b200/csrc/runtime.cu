@@ -23,7 +23,7 @@ static int g_math_mode = initial_math_mode();
 unsigned long long g_launches = 0;
 unsigned long long g_epoch = 0;
 
-static const int kScratchSlots = 10;
+static const int kScratchSlots = 12;
 static void* g_scratch[kScratchSlots] = {nullptr};
 static size_t g_scratch_bytes[kScratchSlots] = {0};
 static unsigned int* g_err_word = nullptr;

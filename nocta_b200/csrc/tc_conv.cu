@@ -1,4 +1,4 @@
-// Halo-resident tensor-core kernels for stride-1 convolutions with filters up to 3 x 3 (plain TF32 mode), sm_100a:
+// Halo-resident tensor-core kernels for stride-1 convolutions with filters up to 3 x 3, sm_100a:
 // TMA-fed tcgen05.mma (kind::tf32), accumulators in tensor memory, inline PTX.
 //
 // An implicit-GEMM convolution that streams one operand tile per filter tap re-reads the same pixels for every tap.  The
@@ -40,6 +40,10 @@
 //                        0..3 pixels = the kW taps of a filter row (kW = 3: three quarters of M useful); B = dY tile;
 //                        one accumulator and one issuing warp per filter row, all kH * kW taps per work item.
 //
+// Channel counts need not be multiples of 32: TMA zero-fills the end of the last chunk and the epilogues drop what lies beyond.
+// Split operands (3xTF32: hi and lo planes, see tc_gemm.cu) lengthen the reduction to three passes over the chunks or pixels with
+// the image or weight-row coordinate moved to the lo plane of one side.
+//
 // Pixel tiles may hang over the image edge: TMA zero-fills what it loads there (which is also the padding) and the
 // epilogues mask what they store.  No cluster launch and no multicast: each CTA loads its own tiles.  Every mbarrier
 // wait is bounded; on expiry the kernel records a code in the device error word, drains, frees its TMEM and returns.
@@ -76,6 +80,8 @@ struct ConvhParams {
     int tiles_m;           // 128-channel tiles (1 when the pixels are on M)
     int kH, kW, pad;
     int cchunks;           // 32-channel chunks of the input channels
+    int passes;            // 1, or 3 over split operands: lo * hi, hi * lo, hi * hi (x * weights)
+    int x_plane, w_plane;  // distance of the lo plane: images of x, rows of the packed weights
     int wrows;             // rows per tap in the packed weights
     int wbox_bytes;        // bytes one weight copy delivers
     int wstages;           // weight ring depth: slots of wslot_bytes in the 96 KB weight region
@@ -155,11 +161,12 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     volatile int* abortp = &abort_flag;
     const int total_tiles = p.tiles_px * p.tiles_m;  // t -> (pixel tile fastest, then channel tile)
     const int ntaps = p.kH * p.kW;
+    const int rchunks = p.cchunks * p.passes;        // reduction chunks of a tile
 
     if (warp == 0) {
         if (lane == 0) {
             // ---------------- producer: halo boxes (one chunk ahead) and weight tiles ----------------
-            int ht = blockIdx.x, hcc = 0;   // cursor of the next halo to request
+            int ht = blockIdx.x, hcc = 0, hpass = 0;   // cursor of the next halo to request
             uint32_t hcount = 0;
             bool ok = true;
             auto issue_halo = [&]() {
@@ -171,17 +178,22 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                 const int th = tt % p.tiles_h, n = tt / p.tiles_h;
                 const uint32_t full = smem_u32(&bar_hfull[slot]);
                 mbar_expect_tx(full, (uint32_t)p.halo_bytes);
-                tma_4d(halo_base + slot * (uint32_t)p.halo_stride, &tmX, hcc * 32, tw * kTW - p.pad, th * kTH - p.pad, DUAL ? 2 * n : n, full);
+                tma_4d(halo_base + slot * (uint32_t)p.halo_stride, &tmX, hcc * 32, tw * kTW - p.pad, th * kTH - p.pad,
+                       (DUAL ? 2 * n : n) + (p.passes == 3 && hpass == 0 ? p.x_plane : 0), full);
                 hcount++;
-                if (++hcc == p.cchunks) { hcc = 0; ht += gridDim.x; }
+                if (++hcc == p.cchunks) {
+                    hcc = 0;
+                    if (++hpass == p.passes) { hpass = 0; ht += gridDim.x; }
+                }
             };
             int s = 0;
             uint32_t ph = 0;
             issue_halo();
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 const int m0 = (t / p.tiles_px) * (PXM ? NCH * 32 : kBM);
-                for (int cc = 0; cc < p.cchunks && ok; cc++) {
-                    int wrow = m0;
+                int cc = 0, pass = 0;
+                for (int rc = 0; rc < rchunks && ok; rc++) {
+                    int wrow = m0 + (p.passes == 3 && pass == 1 ? p.w_plane : 0);
                     for (int t0 = 0; t0 < ntaps && ok; t0 += p.tps) {
                         if (t0 == (ntaps > p.tps ? p.tps : 0)) issue_halo();   // the next chunk's halo, once this chunk is under way
                         if (!ok) break;
@@ -193,6 +205,7 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                             tma_2d(w_base + (uint32_t)(s * p.wslot_bytes + i * p.wbox_bytes), &tmW, cc * 32, wrow, full);
                         if (++s == WS) { s = 0; ph ^= 1u; }
                     }
+                    if (++cc == p.cchunks) { cc = 0; pass++; }
                 }
             }
         }
@@ -225,7 +238,7 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                 tc_fence_after();
                 const uint32_t acc = tmem_base + ab * 256u + (uint32_t)(PXM ? khalf * 128 + iss * NCH * 32 : (DUAL ? iss * 128 : 0));
                 uint32_t acc_started = 0u;   // the first MMA of a tile overwrites the accumulator
-                for (int cc = 0; cc < p.cchunks && ok; cc++, hcount++) {
+                for (int rc = 0; rc < rchunks && ok; rc++, hcount++) {
                     const uint32_t slot = hcount & 1u;
                     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_hfull[slot]), (hcount >> 1) & 1u, p.err, 0x700u + slot, abortp));
                     if (!ok) break;
@@ -476,7 +489,7 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                     fs[ch] = 0.0; fq[ch] = 0.0;
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                for (int c = threadIdx.x - 64; c < NCH * 32; c += 128) {
+                for (int c = threadIdx.x - 64; c < NCH * 32 && m0 + c < p.M; c += 128) {
                     double a = 0.0, b = 0.0;
                     for (int k = 0; k < 4; k++) { a += stat_sh[((k * NCHS + c / 32) * 32 + (c & 31)) * 2]; b += stat_sh[((k * NCHS + c / 32) * 32 + (c & 31)) * 2 + 1]; }
                     double* sd = p.stat + ((size_t)blockIdx.x * p.M + m0 + c) * 2;
@@ -532,13 +545,15 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
                             o.x = __uint_as_float(v[j]);     o.y = __uint_as_float(v[j + 1]);
                             o.z = __uint_as_float(v[j + 2]); o.w = __uint_as_float(v[j + 3]);
                             if (p.bias) {
-                                const float4 b4 = *reinterpret_cast<const float4*>(p.bias + m0 + ch * 32 + j);
-                                o.x += b4.x; o.y += b4.y; o.z += b4.z; o.w += b4.w;
+                                if (m0 + ch * 32 + j < p.M) {   // p.M is a multiple of four
+                                    const float4 b4 = *reinterpret_cast<const float4*>(p.bias + m0 + ch * 32 + j);
+                                    o.x += b4.x; o.y += b4.y; o.z += b4.z; o.w += b4.w;
+                                }
                             }
                             *reinterpret_cast<float4*>(&stat_tile[wq][lane][j]) = o;
                         }
                         __syncwarp();
-                        {
+                        if (m0 + ch * 32 + lane < p.M) {
                             // the warp's 32 pixels: 4 image rows x 8 columns starting at (h0, w0)
                             const int w0 = tw * kTW, h0 = th * kTH + sub * 16 + q * 4;
                             const int wlim = p.Wo - w0, hlim = p.Ho - h0;
@@ -595,11 +610,12 @@ convh_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 // dwh_kernel
 // ------------------------------------------------------------------------------------------
 struct DwhParams {
-    float* partial;        // [splits][Cout][kH * kW * Cin]
-    int Cout, Cin, kH, kW, pad;
+    float* partial;        // [splits][Cout][kH * kW * Cp], Cp = Cin in whole 32-channel chunks
+    int Cout, Cp, kH, kW, pad;
+    int images, passes;    // images of one plane; 1 pass, or 3 over split operands: lo * hi, hi * lo, hi * hi (dy * x)
     int TW, R, PW;         // pixel tile: TW pixels x R image rows per stage; x halo line pitch PW = TW + kW - 1
     int tiles_w, hblocks;  // pixel tiles per image row, row blocks per image
-    int units_total;       // images * hblocks * tiles_w
+    int units_total;       // passes * images * hblocks * tiles_w
     int units_per_split, splits;
     int items;             // work items per split
     int cigs;              // groups of input-channel chunks (item dimension)
@@ -672,21 +688,22 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
                     const int t2 = item / p.kH;
                     ci0 = (t2 % p.cigs) * 128;
                     co0 = (t2 / p.cigs) * 128;
-                    nA = (p.Cout - co0) >= 128 ? 4 : (p.Cout - co0) / 32;
+                    nA = (p.Cout - co0) >= 128 ? 4 : (p.Cout - co0 + 31) / 32;   // chunks beyond Cout: rows never stored
                     nB = 4;
                 } else {
                     kh0 = 0;
                     const int cig = item % p.cigs;
                     ci0 = cig * p.G * 32;
                     co0 = (item / p.cigs) * p.ncol;
-                    nA = (p.Cin / 32 - cig * p.G) < p.G ? (p.Cin / 32 - cig * p.G) : p.G;
-                    nB = p.ncol / 32;
+                    nA = (p.Cp / 32 - cig * p.G) < p.G ? (p.Cp / 32 - cig * p.G) : p.G;
+                    nB = (p.Cout - co0) >= p.ncol ? p.ncol / 32 : (p.Cout - co0 + 31) / 32;   // beyond: columns never stored
                 }
                 const uint32_t bytes = (uint32_t)(nA * p.a_bytes + nB * p.b_bytes);
                 const int u0 = z * p.units_per_split;
                 const int u1 = (u0 + p.units_per_split) < p.units_total ? (u0 + p.units_per_split) : p.units_total;
                 int tw = u0 % p.tiles_w, t3 = u0 / p.tiles_w;
-                int hb = t3 % p.hblocks, n = t3 / p.hblocks;
+                int hb = t3 % p.hblocks, n = t3 / p.hblocks, pass = n / p.images;
+                n -= pass * p.images;
                 for (int u = u0; u < u1; u++) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, p.err, 0x900u + s, abortp)) { ok = false; break; }
                     const uint32_t full = smem_u32(&bar_full[s]);
@@ -694,14 +711,15 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
                     const uint32_t a_dst = tiles_base + (uint32_t)s * (uint32_t)p.stage_bytes;
                     const uint32_t b_dst = a_dst + (uint32_t)(SHIFT ? p.G : 4) * (uint32_t)p.a_stride;
                     const int w0 = tw * p.TW, h0 = hb * p.R;
+                    const int ndy = n + (p.passes == 3 && pass == 0 ? p.images : 0), nx = n + (p.passes == 3 && pass == 1 ? p.images : 0);
                     if (!SHIFT) {
-                        for (int c = 0; c < nA; c++) tma_4d(a_dst + (uint32_t)(c * p.a_stride), &tmDy, co0 + 32 * c, w0, h0, n, full);
-                        for (int c = 0; c < nB; c++) tma_4d(b_dst + (uint32_t)(c * p.b_stride), &tmX, ci0 + 32 * c, w0 - p.pad, h0 + kh0 - p.pad, n, full);
+                        for (int c = 0; c < nA; c++) tma_4d(a_dst + (uint32_t)(c * p.a_stride), &tmDy, co0 + 32 * c, w0, h0, ndy, full);
+                        for (int c = 0; c < nB; c++) tma_4d(b_dst + (uint32_t)(c * p.b_stride), &tmX, ci0 + 32 * c, w0 - p.pad, h0 + kh0 - p.pad, nx, full);
                     } else {
-                        for (int c = 0; c < nA; c++) tma_4d(a_dst + (uint32_t)(c * p.a_stride), &tmX, ci0 + 32 * c, w0 - p.pad, h0 - p.pad, n, full);
-                        for (int c = 0; c < nB; c++) tma_4d(b_dst + (uint32_t)(c * p.b_stride), &tmDy, co0 + 32 * c, w0, h0, n, full);
+                        for (int c = 0; c < nA; c++) tma_4d(a_dst + (uint32_t)(c * p.a_stride), &tmX, ci0 + 32 * c, w0 - p.pad, h0 - p.pad, nx, full);
+                        for (int c = 0; c < nB; c++) tma_4d(b_dst + (uint32_t)(c * p.b_stride), &tmDy, co0 + 32 * c, w0, h0, ndy, full);
                     }
-                    if (++tw == p.tiles_w) { tw = 0; if (++hb == p.hblocks) { hb = 0; n++; } }
+                    if (++tw == p.tiles_w) { tw = 0; if (++hb == p.hblocks) { hb = 0; if (++n == p.images) { n = 0; pass++; } } }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
@@ -736,7 +754,7 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
                 int nA = 1;
                 if (SHIFT) {
                     const int cig = item % p.cigs;
-                    nA = (p.Cin / 32 - cig * p.G) < p.G ? (p.Cin / 32 - cig * p.G) : p.G;
+                    nA = (p.Cp / 32 - cig * p.G) < p.G ? (p.Cp / 32 - cig * p.G) : p.G;
                 }
                 const int u0 = z * p.units_per_split;
                 const int u1 = (u0 + p.units_per_split) < p.units_total ? (u0 + p.units_per_split) : p.units_total;
@@ -777,7 +795,7 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
         const int q = warp & 3;
         const int r = q * 32 + lane;
         const int ntaps = p.kH * p.kW;
-        const size_t row_len = (size_t)ntaps * p.Cin;
+        const size_t row_len = (size_t)ntaps * p.Cp;
         uint32_t work_iter = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < total_work; w += gridDim.x, work_iter++) {
@@ -794,7 +812,7 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
                 const int ci0 = (t2 % p.cigs) * 128, co = (t2 / p.cigs) * 128 + r;
                 const bool co_ok = co < p.Cout;
                 for (int kw = 0; kw < p.kW; kw++) {
-                    float* dst = pz + (size_t)co * row_len + (size_t)(kh0 * p.kW + kw) * p.Cin + ci0;
+                    float* dst = pz + (size_t)co * row_len + (size_t)(kh0 * p.kW + kw) * p.Cp + ci0;
 #pragma unroll 1
                     for (int c0 = 0; c0 < 128; c0 += 32) {
                         uint32_t v[32];
@@ -812,19 +830,21 @@ dwh_kernel(const __grid_constant__ CUtensorMap tmDy, const __grid_constant__ CUt
                 // lane r = (pixel shift kw = q, input channel lane); columns = output channels
                 const int cig = item % p.cigs;
                 const int co0 = (item / p.cigs) * p.ncol;
-                const int nA = (p.Cin / 32 - cig * p.G) < p.G ? (p.Cin / 32 - cig * p.G) : p.G;
+                const int nA = (p.Cp / 32 - cig * p.G) < p.G ? (p.Cp / 32 - cig * p.G) : p.G;
                 if (q < p.kW) {
                     for (int g = 0; g < nA; g++) {
                         const int ci = (cig * p.G + g) * 32 + lane;
                         for (int kh = 0; kh < p.kH; kh++) {
-                            float* dst = pz + (size_t)co0 * row_len + (size_t)(kh * p.kW + q) * p.Cin + ci;
+                            float* dst = pz + (size_t)co0 * row_len + (size_t)(kh * p.kW + q) * p.Cp + ci;
 #pragma unroll 1
                             for (int c0 = 0; c0 < p.ncol; c0 += 32) {
                                 uint32_t v[32];
                                 tmem_ld32(acc + (uint32_t)((g * p.kH + kh) * p.ncol + c0), v);
                                 tmem_ld_wait();
+                                const int lim = p.Cout - co0 - c0;
 #pragma unroll
-                                for (int j = 0; j < 32; j++) dst[(size_t)(c0 + j) * row_len] = __uint_as_float(v[j]);
+                                for (int j = 0; j < 32; j++)
+                                    if (j < lim) dst[(size_t)(c0 + j) * row_len] = __uint_as_float(v[j]);
                             }
                         }
                     }
@@ -888,29 +908,28 @@ static int convh_launch(const CUtensorMap& tw, const CUtensorMap& tx, ConvhParam
 }
 
 int conv_halo_nhwc(float* y, const float* x, const float* wpacked, const float* bias, int N, int H, int W, int Cin, int Cout,
-                   int kH, int kW, int pad, int mode, cudaStream_t st) {
+                   int kH, int kW, int pad, int planes, cudaStream_t st) {
     const int Ho = H + 2 * pad - kH + 1, Wo = W + 2 * pad - kW + 1;
-    if (mode != NC_CUDA_MATH_TF32) return NC_CUDA_ERR_UNSUPPORTED;   // no operand-conversion stage in this kernel
     if (kH < 1 || kW < 1 || kH > 3 || kW > 3 || Ho <= 0 || Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((Cin % 32) || (Cout % 4) || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
+    if ((Cin % 4) || (Cout % 4) || Cin < 16 || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
     if ((long long)N * Ho * Wo * Cout >= 0x7fffffffLL) return NC_CUDA_ERR_UNSUPPORTED;
     // Tiles are 8 pixels wide and up to 32 high.  With the channels on M one thread issues all MMAs of a tile, which
     // only keeps the tensor pipe busy with N = 8 * rows = 256.  Images of exactly 16 rows go two to a tile (DUAL, channels on
     // M only); other images lower than 24 rows run faster on the per-tap kernel, whose 256-pixel boxes span several images.
-    const bool dual = Ho == 16 && (N % 2 == 0) && !(Cout % 32 == 0 && Cout <= 96);
+    const bool dual = Ho == 16 && (N % 2 == 0) && Cout > 96;
     if (Ho < 24 && !dual) return NC_CUDA_ERR_UNSUPPORTED;
     // Pixels on M for up to 96 output channels (measured on the 64-channel 64 x 64 layer at batch 256: 447 against 344
     // TFLOP/s with the channels on M); from 128 channels on, channels on M with N = 256 pixels is the faster shape
     // (698 against 636 TFLOP/s on the 128-channel 32 x 32 layer).
-    const int ncol = Cout;
-    const bool pxm = (Cout % 32 == 0) && Cout <= 96 && (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15u) == 0) &&
+    const int ncol = (Cout + 31) & ~31;
+    const bool pxm = Cout <= 96 && (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15u) == 0) &&
                      (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
     CUtensorMap tw, tx;
-    unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout};
+    unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout * planes};
     unsigned long long ws[1] = {(unsigned long long)Cin};
     unsigned wb[2] = {32, (unsigned)(pxm ? ncol : 128)};
     if (!make_map(&tw, wpacked, 2, wd, ws, wb, false)) return NC_CUDA_ERR_UNSUPPORTED;
-    unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N};
+    unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N * planes};
     unsigned long long str[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
     unsigned box[4] = {32, (unsigned)(kTW + kW - 1), (unsigned)(dual ? Ho + kH - 1 : kTH + kH - 1), dual ? 2u : 1u};
     if (!make_map(&tx, x, 4, dims, str, box, false)) return NC_CUDA_ERR_UNSUPPORTED;
@@ -920,9 +939,11 @@ int conv_halo_nhwc(float* y, const float* x, const float* wpacked, const float* 
     p.tiles_w = (Wo + kTW - 1) / kTW; p.tiles_h = (p.Ho + kTH - 1) / kTH;
     p.tiles_px = (dual ? N / 2 : N) * p.tiles_w * p.tiles_h;
     p.half_rows = Ho + kH - 1;
-    p.tiles_m = pxm ? Cout / ncol : (Cout + kBM - 1) / kBM;
+    p.tiles_m = pxm ? 1 : (Cout + kBM - 1) / kBM;
     p.kH = kH; p.kW = kW; p.pad = pad;
-    p.cchunks = Cin / 32;
+    p.cchunks = (Cin + 31) / 32;
+    p.passes = planes == 2 ? 3 : 1;
+    p.x_plane = N; p.w_plane = kH * kW * Cout;
     p.wrows = Cout;
     p.wbox_bytes = (pxm ? ncol : 128) * 128;
     // Taps per weight stage: as many as leave two stages in the 96 KB weight region, spread evenly over the stages of a
@@ -983,15 +1004,16 @@ static bool pick_dw_tile(int Wo, int Ho, int kW, int halo_rows, int nchunk_dy, i
 }
 
 int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W, int Cin, int Cout, int kH, int kW, int pad,
-                      int mode, cudaStream_t st) {
+                      int planes, cudaStream_t st) {
     const int Ho = H + 2 * pad - kH + 1, Wo = W + 2 * pad - kW + 1;
-    if (mode != NC_CUDA_MATH_TF32) return NC_CUDA_ERR_UNSUPPORTED;
     if (kH < 1 || kW < 2 || kH > 3 || kW > 3 || Ho <= 0 || Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((Cin % 32) || (Cout % 32)) return NC_CUDA_ERR_UNSUPPORTED;
+    if ((Cin % 4) || (Cout % 4) || Cin < 16 || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
     if ((long long)N * Ho * Wo < 4096) return NC_CUDA_ERR_UNSUPPORTED;   // too few pixels to split over the GPU
     const bool shift = (Cin % 128) != 0;
     DwhParams p = {};
-    p.Cout = Cout; p.Cin = Cin; p.kH = kH; p.kW = kW; p.pad = pad;
+    const int Cp = (Cin + 31) & ~31;
+    p.Cout = Cout; p.Cp = Cp; p.kH = kH; p.kW = kW; p.pad = pad;
+    p.images = N; p.passes = planes == 2 ? 3 : 1;
     int dy_stride = 0, x_stride = 0;
     if (!shift) {
         p.ncol = 128; p.G = 4;
@@ -1001,11 +1023,15 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
         p.a_stride = dy_stride; p.b_stride = x_stride;
     } else {
         // one accumulator per (input chunk, filter row): kH * G * ncol <= 512 columns
-        p.ncol = Cout >= 128 ? 128 : Cout;            // Cout % 32 == 0: 32, 64, 96 or 128
-        if (Cout > 128 && Cout % 128) return NC_CUDA_ERR_UNSUPPORTED;
-        p.G = (kH * 2 * p.ncol <= 512 && Cin >= 64) ? 2 : 1;
-        p.cigs = (Cin / 32 + p.G - 1) / p.G;
-        p.items = (Cout / p.ncol) * p.cigs;
+        // an MMA costs max(N / 2, 48) cycles: the width with the cheapest set of tiles over Cout, narrower on a tie
+        int best = 1 << 30;
+        for (int nc = 32; nc <= 128; nc += 32) {
+            const int cost = (Cout + nc - 1) / nc * (nc / 2 > 48 ? nc / 2 : 48);
+            if (cost < best) { best = cost; p.ncol = nc; }
+        }
+        p.G = (kH * 2 * p.ncol <= 512 && Cp >= 64) ? 2 : 1;
+        p.cigs = (Cp / 32 + p.G - 1) / p.G;
+        p.items = ((Cout + p.ncol - 1) / p.ncol) * p.cigs;
         // two large stages beat three smaller ones here (measured: 64 -> 64 at 64 x 64 184 -> 173 us, 64 -> 128 at 32 x 32
         // 83 -> 75 us; the other variant loses 10 % with two): three issuing warps stop at every stage barrier together
         if (!pick_dw_tile(Wo, Ho, kW, kH - 1, p.ncol / 32, p.G, 2, &p.TW, &p.R, &p.stage_bytes, &dy_stride, &x_stride)) return NC_CUDA_ERR_UNSUPPORTED;
@@ -1015,7 +1041,7 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
     p.nissue = shift ? kH : kW;
     p.tiles_w = (Wo + p.TW - 1) / p.TW;
     p.hblocks = (Ho + p.R - 1) / p.R;
-    p.units_total = N * p.hblocks * p.tiles_w;
+    p.units_total = p.passes * N * p.hblocks * p.tiles_w;
     const int dy_bytes = p.TW * p.R * 128, x_bytes = p.PW * (p.R + (shift ? kH - 1 : 0)) * 128;
     p.a_bytes = shift ? x_bytes : dy_bytes;
     p.b_bytes = shift ? dy_bytes : x_bytes;
@@ -1028,18 +1054,18 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
     if (splits > p.units_total / 4) splits = p.units_total / 4 > 0 ? p.units_total / 4 : 1;
     p.units_per_split = (p.units_total + splits - 1) / splits;
     p.splits = (p.units_total + p.units_per_split - 1) / p.units_per_split;
-    const size_t partial_bytes = sizeof(float) * (size_t)p.splits * Cout * kH * kW * Cin;
+    const size_t partial_bytes = sizeof(float) * (size_t)p.splits * Cout * kH * kW * Cp;
     if (partial_bytes > (size_t)512 << 20) return NC_CUDA_ERR_UNSUPPORTED;
     p.partial = (float*)ncc::scratch(2, partial_bytes, st);
     if (!p.partial) return NC_CUDA_ERR_RUNTIME;
     p.err = ncc::device_error_word();
     CUtensorMap tdy, tx;
     {
-        unsigned long long dims[4] = {(unsigned long long)Cout, (unsigned long long)Wo, (unsigned long long)Ho, (unsigned long long)N};
+        unsigned long long dims[4] = {(unsigned long long)Cout, (unsigned long long)Wo, (unsigned long long)Ho, (unsigned long long)N * planes};
         unsigned long long str[3] = {(unsigned long long)Cout, (unsigned long long)Wo * Cout, (unsigned long long)Ho * Wo * Cout};
         unsigned box[4] = {32, (unsigned)p.TW, (unsigned)p.R, 1};
         if (!make_map(&tdy, dy, 4, dims, str, box, true)) return NC_CUDA_ERR_UNSUPPORTED;
-        unsigned long long xd[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N};
+        unsigned long long xd[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N * planes};
         unsigned long long xs[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
         unsigned xbox[4] = {32, (unsigned)p.PW, (unsigned)(p.R + (shift ? kH - 1 : 0)), 1};
         if (!make_map(&tx, x, 4, xd, xs, xbox, true)) return NC_CUDA_ERR_UNSUPPORTED;

@@ -1,6 +1,6 @@
-// Tensor-core contractions for sm_100a: TMA-fed, tcgen05.mma (kind::tf32) with the accumulator in
+// Tensor-core contractions for sm_100a: TMA-fed tcgen05.mma (kind::tf32) with the accumulator in
 // tensor memory, written with inline PTX.  tc_kernel serves four problem kinds; the halo-resident convolution and
-// weight-gradient kernels, which take the stride-1 filters up to 3 x 3 in plain TF32 mode, live in tc_conv.cu.
+// weight-gradient kernels, which take the stride-1 filters up to 3 x 3, live in tc_conv.cu.
 //
 //   GEMM   D(M,N) = A * B^T        either operand K-major or MN-major in memory
 //   CONV   channels-last implicit GEMM, stride 1: rows = 128 output pixels (a w x h x n box),
@@ -13,13 +13,18 @@
 //          tcgen05.mma (kind::tf32, one CTA) takes max(N / 2, operand bytes / 128, about 46) cycles
 //          whatever M is, so M = 128 with N >= 128 is the full-rate shape; with pixels on N that holds
 //          for any channel count >= 128, while few channels on N (N = 64: 48 cycles) would not.
+//          Strided layers: the forward box is a TMA box with traversal stride; the input gradient is one
+//          stride-1 convolution per residue class of the input coordinates (ConvClass), all in one launch.
 //   DW     weight gradient: rows = output channels, cols = (kh, kw, ci), reduction = 32-pixel
 //          boxes; both operands MN-major; split over the reduction with an ordered second stage.
 //
+// The kernel multiplies TF32 operands as they lie in memory.  The accuracy modes are prepared in memory: operands rounded to
+// nearest TF32, or for 3xTF32 split into two planes hi and lo (split_operand), and the reduction then runs over three passes,
+// lo * hi, hi * lo, hi * hi: to the kernel a reduction three times as long with other tile coordinates.  The small products come
+// first, so the accumulator is rounded at full size only by the last third of the additions.
+//
 // CTA = 6 warps (kernels with an MN-major operand add up to five more TMA-issuing warps): warp 0 issues TMA, warp 1
-// allocates TMEM and issues MMAs (one lane), warps 2-5
-// convert operands in shared memory when the math mode asks for it (round-to-nearest TF32, or the
-// hi/lo split of 3xTF32) and then run the epilogue (tcgen05.ld -> registers -> global).
+// allocates TMEM and issues MMAs (one lane), warps 2-5 run the epilogue (tcgen05.ld -> registers -> global).
 // Every mbarrier wait is bounded: on expiry the kernel records a code in the device error word,
 // drains, frees its TMEM and returns.
 //
@@ -32,9 +37,22 @@ namespace tc {
 
 enum { KIND_GEMM = 0, KIND_CONV = 1, KIND_DW = 2, KIND_CONVT = 3 };
 
+// One stride-1 convolution of a CONVT launch: taps, paddings, where its weights start, its output extent and where that lies
+// in the output tensor (stride and offset per axis).
+struct ConvClass {
+    int kH, kW, pad_h, pad_w;
+    int wrow0;               // first row of its packed weights
+    int Ho, Wo, tiles_w, tiles_h;
+    int oh0, ow0;            // output pixel (h, w) of the class = (oh0 + os * h, ow0 + os * w) of the tensor
+    int tile0;               // first pixel tile
+};
+constexpr int kMaxClasses = 4;
+
 struct TcParams {
     int kind;
     int M, N;              // logical output extent (store masks)
+    int passes, pass_tiles;// reduction passes (1, or 3 over split operands) of pass_tiles tiles each
+    int a_plane, b_plane;  // coordinate distance of the lo plane of A and B (rows, or images)
     int num_k_tiles;       // reduction tiles in total
     int k_tiles_per_split; // reduction tiles per blockIdx.z
     float* D;
@@ -47,12 +65,16 @@ struct TcParams {
     int tiles_w, tiles_h;
     int Ho, Wo, Nimg;
     int kW, pad;
+    int stride;            // CONVT, DW: pixel stride of the input box
     int cchunks;           // CONV: 32-channel chunks of the reduction channels
     int wrows;             // CONV: rows per (kh,kw) block of the packed weights (= output channels)
-    int Cin;               // DW: input channels (column index -> (shift, ci))
+    int Cin;               // DW: input channels, padded to whole chunks (column index -> (shift, ci))
     int lbw, lbh;                  // CONVT: log2 of the pixel box width / height
     int tiles_m, tiles_n, splits;  // persistent tile walk
     int stages;                    // operand ring depth
+    // CONVT
+    int classes, os, Hout, Wout;   // residue classes; output pixel stride and tensor extent
+    ConvClass cls[kMaxClasses];
     double* stat;                  // CONVT, non-null: per CTA and channel (sum, sum of squares) of the output it wrote, [gridDim.x][M][2]
     unsigned int* err;
     double flops;                  // host only: algorithmic FLOPs of the launch, for the profiling scope
@@ -68,23 +90,19 @@ constexpr int CHUNK_BYTES = 32 * BK * 4;  // one 32 x 32 MN-major chunk: 4 KB
 constexpr int kMaxStages = 8;
 constexpr int kSmemBudget = 196 * 1024;  // one persistent CTA per SM
 
-template <int BN, int MODE>
+// NACC accumulators take the k-steps in turn and are added in f32 by the epilogue: the 3xTF32 GEMM spreads its additions over two,
+// because the tensor core's own accumulation is the largest error term left in that mode.
+template <int BN, int NACC>
 struct TileCfg {
     static constexpr int B_BYTES = BN * BK * 4;
-    static constexpr int OPER_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGE_BYTES = OPER_BYTES * (MODE == 2 ? 2 : 1);
+    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int STAGES_RAW = kSmemBudget / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > kMaxStages ? kMaxStages : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + alignment slack
     static constexpr int ACC_COLS = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
-    // 3xTF32 spreads the reduction over several accumulators (round-robin per k-step) and adds them
-    // in FP32 in the epilogue: the tensor core's own accumulation is the largest error term left in
-    // that mode and it grows with the number of additions into one accumulator.
-    static constexpr int NACC = MODE == 2 ? (512 / ACC_COLS > 4 ? 4 : 512 / ACC_COLS) : 1;
-    // plain TF32 keeps two accumulator buffers so the epilogue of one tile overlaps the MMAs of the next;
-    // the converting modes use the epilogue warps during the main loop, so one buffer is enough there
-    static constexpr int NBUF = MODE == 0 ? 2 : 1;
+    static constexpr int NBUF = 2;   // the epilogue of one tile overlaps the MMAs of the next
     static constexpr int TMEM_COLS = ACC_COLS * NACC * NBUF;
+    static_assert(TMEM_COLS <= 512, "tensor memory");
 };
 
 // MN-major operands arrive as one copy per 32-wide chunk (up to 12 per stage) and a thread spends on the
@@ -100,30 +118,51 @@ struct ProdCfg {
     static constexpr int THREADS = 192 + 32 * (NPROD - 1);
 };
 
-template <int BN, bool A_MN, bool B_MN, int MODE>
+// What a CTA does for tile t of its walk
+struct Tile {
+    int m0, n_tile, z, kt_begin, kt_end, cls, px;   // cls, px: CONVT residue class and pixel tile within it
+};
+__device__ __forceinline__ Tile tile_of(const TcParams& p, int t) {
+    Tile o;
+    o.n_tile = t % p.tiles_n;
+    const int r = t / p.tiles_n;
+    o.m0 = (r % p.tiles_m) * BM;
+    o.z = r / p.tiles_m;
+    o.kt_begin = o.z * p.k_tiles_per_split;
+    o.kt_end = o.kt_begin + p.k_tiles_per_split;
+    if (o.kt_end > p.num_k_tiles) o.kt_end = p.num_k_tiles;
+    o.cls = 0;
+    o.px = o.n_tile;
+    if (p.kind == KIND_CONVT) {
+        while (o.cls + 1 < p.classes && o.n_tile >= p.cls[o.cls + 1].tile0) o.cls++;
+        o.px = o.n_tile - p.cls[o.cls].tile0;
+        o.kt_end = p.cls[o.cls].kH * p.cls[o.cls].kW * p.cchunks * p.passes;   // never split
+    }
+    return o;
+}
+
+template <int BN, bool A_MN, bool B_MN, int NACC>
 __global__ void __launch_bounds__(352, 1)
-tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcParams p) {
-    using Cfg = TileCfg<BN, MODE>;
-    constexpr int NBUF = Cfg::NBUF;  // accumulator buffers in tensor memory (2 = epilogue overlaps the next tile)
+tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TcParams p) {
+    using Cfg = TileCfg<BN, NACC>;
+    constexpr int NBUF = Cfg::NBUF;
     const int STAGES = p.stages;
     extern __shared__ uint8_t dyn_smem[];
     __shared__ __align__(8) uint64_t bar_full[kMaxStages];
     __shared__ __align__(8) uint64_t bar_empty[kMaxStages];
-    __shared__ __align__(8) uint64_t bar_conv[kMaxStages];
     __shared__ __align__(8) uint64_t bar_acc_full[2];
     __shared__ __align__(8) uint64_t bar_acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
+    __shared__ __align__(16) float turn[4][32][36];   // per epilogue warp: a 32 x 32 block between accumulator and store
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t tiles_base = (smem_u32(dyn_smem) + 1023u) & ~1023u;
-    uint8_t* tiles_generic = dyn_smem + (tiles_base - smem_u32(dyn_smem));
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
             mbar_init(smem_u32(&bar_full[s]), (uint32_t)ProdCfg<A_MN, B_MN, BN>::NPROD);
             mbar_init(smem_u32(&bar_empty[s]), 1);
-            mbar_init(smem_u32(&bar_conv[s]), 128);
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(smem_u32(&bar_acc_full[b]), 1);
@@ -167,22 +206,20 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             uint32_t ph = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-                const int n_tile = t % p.tiles_n, r_ = t / p.tiles_n, m_tile = r_ % p.tiles_m, z = r_ / p.tiles_m;
-                const int kt_begin = z * p.k_tiles_per_split;
-                int kt_end = kt_begin + p.k_tiles_per_split;
-                if (kt_end > p.num_k_tiles) kt_end = p.num_k_tiles;
-                const int m0 = m_tile * BM, n0 = n_tile * BN;
+                const Tile T = tile_of(p, t);
+                const int m0 = T.m0, n0 = T.n_tile * BN;
                 const int edge = forA ? p.M - m0 : p.N - n0;  // chunks starting at or beyond it are skipped
                 int my_n = 0;                                 // copies this producer issues per stage of this tile
                 for (int c = own; c < (forA ? NACH : NBCH); c += step) my_n += (32 * c < edge) ? 1 : 0;
                 const bool chunked = forA ? A_MN : B_MN;
                 const uint32_t my_bytes = chunked ? (uint32_t)my_n * CHUNK_BYTES : (forA ? (uint32_t)A_BYTES : (uint32_t)Cfg::B_BYTES);
+                int pass = T.kt_begin / p.pass_tiles, lk = T.kt_begin - pass * p.pass_tiles;
                 int dtw = 0, dth = 0, dtn = 0;
                 // DW: (first channel, tap) of this producer's B chunks
                 int ci0[4] = {0, 0, 0, 0}, dkh[4] = {0, 0, 0, 0}, dkw[4] = {0, 0, 0, 0};
                 if (p.kind == KIND_DW) {
-                    dtw = kt_begin % p.tiles_w;
-                    const int tt = kt_begin / p.tiles_w;
+                    dtw = lk % p.tiles_w;
+                    const int tt = lk / p.tiles_w;
                     dth = tt % p.tiles_h; dtn = tt / p.tiles_h;
                     if (!forA) {
 #pragma unroll
@@ -194,37 +231,39 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                         }
                     }
                 }
-                for (int kt = kt_begin; kt < kt_end; kt++) {
+                for (int kt = T.kt_begin; kt < T.kt_end; kt++) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, p.err, 0x100u + s, abortp)) { ok = false; break; }
                     const uint32_t full = smem_u32(&bar_full[s]);
                     const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES;
                     const uint32_t b_dst = a_dst + A_BYTES;
+                    // split operands: passes lo * hi, hi * lo, hi * hi
+                    const int off = p.passes == 1 ? 0 : (forA ? (pass == 0 ? p.a_plane : 0) : (pass == 1 ? p.b_plane : 0));
                     if (my_bytes == 0) {
                         mbar_arrive(full);
                     } else {
                         mbar_expect_tx(full, my_bytes);
                         if (p.kind == KIND_GEMM) {
-                            const int k0 = kt * BK;
+                            const int k0 = lk * BK;
                             if (forA) {
-                                if (!A_MN) tma_2d(a_dst, &tmA, k0, m0, full);
+                                if (!A_MN) tma_2d(a_dst, &tmA, k0, m0 + off, full);
                                 else {
 #pragma unroll
                                     for (int i = 0; i < 4; i++) {
                                         const int c = own + i * step;
-                                        if (c < NACH && 32 * c < edge) tma_2d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, k0, full);
+                                        if (c < NACH && 32 * c < edge) tma_2d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, k0 + off, full);
                                     }
                                 }
                             } else if (!B_MN) {
-                                tma_2d(b_dst, &tmB, k0, n0, full);
+                                tma_2d(b_dst, &tmB, k0, n0 + off, full);
                             } else {
 #pragma unroll
                                 for (int i = 0; i < 4; i++) {
                                     const int c = own + i * step;
-                                    if (c < NBCH && 32 * c < edge) tma_2d(b_dst + c * CHUNK_BYTES, &tmB, n0 + 32 * c, k0, full);
+                                    if (c < NBCH && 32 * c < edge) tma_2d(b_dst + c * CHUNK_BYTES, &tmB, n0 + 32 * c, k0 + off, full);
                                 }
                             }
                         } else {  // KIND_DW (both operands MN-major)
-                            const int w0 = dtw * p.bw, h0 = dth * p.bh, nn0 = dtn * p.bn;
+                            const int w0 = dtw * p.bw, h0 = dth * p.bh, nn0 = dtn * p.bn + off;
                             if (forA) {
 #pragma unroll
                                 for (int i = 0; i < 4; i++) {
@@ -235,7 +274,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 #pragma unroll
                                 for (int i = 0; i < 4; i++) {
                                     const int c = own + i * step;
-                                    if (c < NBCH && 32 * c < edge) tma_4d(b_dst + c * CHUNK_BYTES, &tmB, ci0[i], w0 + dkw[i] - p.pad, h0 + dkh[i] - p.pad, nn0, full);
+                                    if (c < NBCH && 32 * c < edge)
+                                        tma_4d(b_dst + c * CHUNK_BYTES, &tmB, ci0[i], w0 * p.stride + dkw[i] - p.pad, h0 * p.stride + dkh[i] - p.pad, nn0, full);
                                 }
                             }
                         }
@@ -243,6 +283,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                     if (p.kind == KIND_DW) {
                         if (++dtw == p.tiles_w) { dtw = 0; if (++dth == p.tiles_h) { dth = 0; dtn++; } }
                     }
+                    if (++lk == p.pass_tiles) { lk = 0; pass++; dtw = 0; dth = 0; dtn = 0; }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
@@ -256,73 +297,50 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             uint32_t ph = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-                const int n_tile = t % p.tiles_n, r_ = t / p.tiles_n, m_tile = r_ % p.tiles_m, z = r_ / p.tiles_m;
-                const int kt_begin = z * p.k_tiles_per_split;
-                int kt_end = kt_begin + p.k_tiles_per_split;
-                if (kt_end > p.num_k_tiles) kt_end = p.num_k_tiles;
-                const int m0 = m_tile * BM, n0 = n_tile * BN;
-                // pixel box of this tile (CONV: the m tile, CONVT: the n tile)
-                int pw0 = 0, ph0 = 0, pn0 = 0;
-                if (p.kind == KIND_CONV || p.kind == KIND_CONVT) {
-                    const int pt = p.kind == KIND_CONV ? m_tile : n_tile;
-                    const int tw = pt % p.tiles_w, tt = pt / p.tiles_w;
-                    pw0 = tw * p.bw; ph0 = (tt % p.tiles_h) * p.bh; pn0 = (tt / p.tiles_h) * p.bn;
+                const Tile T = tile_of(p, t);
+                const int m0 = T.m0, n0 = T.n_tile * BN;
+                int pass = 0, lk = 0;
+                // pixel box of this tile (CONV: the m tile, CONVT: the n tile), running (tap, chunk)
+                int pw0 = 0, ph0 = 0, pn0 = 0, cc = 0, kh = 0, kw = 0, shift = 0, kWc = p.kW, taps_left = 0, wrow0 = 0, taps = 0;
+                if (p.kind == KIND_CONV) {
+                    const int pt = m0 / BM, tw = pt % p.tiles_w, tt = pt / p.tiles_w;
+                    pw0 = tw * p.bw - p.pad; ph0 = (tt % p.tiles_h) * p.bh - p.pad; pn0 = (tt / p.tiles_h) * p.bn;
+                    taps = p.pass_tiles / p.cchunks;
+                } else if (p.kind == KIND_CONVT) {
+                    const ConvClass& c = p.cls[T.cls];
+                    const int tw = T.px % c.tiles_w, tt = T.px / c.tiles_w;
+                    pw0 = tw * p.bw * p.stride - c.pad_w; ph0 = (tt % c.tiles_h) * p.bh * p.stride - c.pad_h; pn0 = (tt / c.tiles_h) * p.bn;
+                    kWc = c.kW; wrow0 = c.wrow0;
+                    taps = c.kH * c.kW;
+                } else {
+                    pass = T.kt_begin / p.pass_tiles; lk = T.kt_begin - pass * p.pass_tiles;
                 }
-                // running decomposition of kt: CONV/CONVT (tap kh,kw ; chunk cc), DW (box tw,th,tn)
-                int cc = 0, kh = 0, kw = 0, shift = 0, dtw = 0, dth = 0, dtn = 0, dw_ci0 = 0, dw_kh0 = 0, dw_kw0 = 0;
-                if (p.kind == KIND_CONV || p.kind == KIND_CONVT) {
-                    shift = kt_begin / p.cchunks; cc = kt_begin - shift * p.cchunks;
-                    kh = shift / p.kW; kw = shift - kh * p.kW;
-                } else if (p.kind == KIND_DW) {
-                    dtw = kt_begin % p.tiles_w;
-                    const int tt = kt_begin / p.tiles_w;
-                    dth = tt % p.tiles_h; dtn = tt / p.tiles_h;
-                    const int dshift = n0 / p.Cin;
-                    dw_ci0 = n0 - dshift * p.Cin;
-                    dw_kh0 = dshift / p.kW; dw_kw0 = dshift - dw_kh0 * p.kW;
-                }
-                for (int kt = kt_begin; kt < kt_end; kt++) {
+                taps_left = taps;
+                for (int kt = T.kt_begin; kt < T.kt_end; kt++) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, p.err, 0x100u + s, abortp)) { ok = false; break; }
                     const uint32_t full = smem_u32(&bar_full[s]);
-                    mbar_expect_tx(full, (uint32_t)Cfg::OPER_BYTES);
+                    mbar_expect_tx(full, (uint32_t)Cfg::STAGE_BYTES);
                     const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES;
                     const uint32_t b_dst = a_dst + A_BYTES;
+                    const int offA = (p.passes == 3 && pass == 0) ? p.a_plane : 0, offB = (p.passes == 3 && pass == 1) ? p.b_plane : 0;
                     if (p.kind == KIND_GEMM) {
-                        const int k0 = kt * BK;
-                        if (!A_MN) {
-                            tma_2d(a_dst, &tmA, k0, m0, full);
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < BM / 32; c++) tma_2d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, k0, full);
-                        }
-                        if (!B_MN) {
-                            tma_2d(b_dst, &tmB, k0, n0, full);
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < BN / 32; c++) tma_2d(b_dst + c * CHUNK_BYTES, &tmB, n0 + 32 * c, k0, full);
-                        }
-                    } else if (p.kind == KIND_CONV) {
-                        tma_4d(a_dst, &tmA, cc * 32, pw0 + kw - p.pad, ph0 + kh - p.pad, pn0, full);
-                        tma_2d(b_dst, &tmB, cc * 32, shift * p.wrows + n0, full);
-                    } else if (p.kind == KIND_CONVT) {
-                        tma_2d(a_dst, &tmA, cc * 32, shift * p.wrows + m0, full);
-                        tma_4d(b_dst, &tmB, cc * 32, pw0 + kw - p.pad, ph0 + kh - p.pad, pn0, full);
+                        const int k0 = lk * BK;
+                        tma_2d(a_dst, &tmA, k0, m0 + offA, full);
+                        tma_2d(b_dst, &tmB, k0, n0 + offB, full);
+                        if (++lk == p.pass_tiles) { lk = 0; pass++; }
                     } else {
-                        const int w0 = dtw * p.bw, h0 = dth * p.bh, nn0 = dtn * p.bn;
-#pragma unroll
-                        for (int c = 0; c < BM / 32; c++) tma_4d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, w0, h0, nn0, full);
-                        // column chunk c covers columns n0 + 32c .. : (tap, ci0) advance by 32 channels per chunk
-                        int ci0 = dw_ci0, dkh = dw_kh0, dkw = dw_kw0;
-#pragma unroll
-                        for (int c = 0; c < BN / 32; c++) {
-                            tma_4d(b_dst + c * CHUNK_BYTES, &tmB, ci0, w0 + dkw - p.pad, h0 + dkh - p.pad, nn0, full);
-                            ci0 += 32;
-                            if (ci0 >= p.Cin) { ci0 = 0; if (++dkw == p.kW) { dkw = 0; dkh++; } }
+                        if (p.kind == KIND_CONV) {
+                            tma_4d(a_dst, &tmA, cc * 32, pw0 + kw, ph0 + kh, pn0 + offA, full);
+                            tma_2d(b_dst, &tmB, cc * 32, shift * p.wrows + n0 + offB, full);
+                        } else {
+                            tma_2d(a_dst, &tmA, cc * 32, wrow0 + shift * p.wrows + m0 + offA, full);
+                            tma_4d(b_dst, &tmB, cc * 32, pw0 + kw, ph0 + kh, pn0 + offB, full);
                         }
-                        if (++dtw == p.tiles_w) { dtw = 0; if (++dth == p.tiles_h) { dth = 0; dtn++; } }
-                    }
-                    if (p.kind == KIND_CONV || p.kind == KIND_CONVT) {
-                        if (++cc == p.cchunks) { cc = 0; shift++; if (++kw == p.kW) { kw = 0; kh++; } }
+                        if (++cc == p.cchunks) {
+                            cc = 0; shift++;
+                            if (++kw == kWc) { kw = 0; kh++; }
+                            if (--taps_left == 0) { taps_left = taps; shift = 0; kh = 0; kw = 0; pass++; }
+                        }
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
@@ -354,42 +372,27 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             // the top of the next round is skipped.
             bool known_ready = false;
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, tile_iter++) {
-                const int z = (t / p.tiles_n) / p.tiles_m;
-                const int kt_begin = z * p.k_tiles_per_split;
-                int kt_end = kt_begin + p.k_tiles_per_split;
-                if (kt_end > p.num_k_tiles) kt_end = p.num_k_tiles;
-                const int nk = kt_end - kt_begin;
+                const Tile T = tile_of(p, t);
+                const int nk = T.kt_end - T.kt_begin;
                 const uint32_t ab = tile_iter % NBUF;
                 // wait until the epilogue has drained this accumulator buffer (first use passes at once)
                 if (!mbar_wait(smem_u32(&bar_acc_empty[ab]), ((tile_iter / NBUF) & 1u) ^ 1u, p.err, 0x500u + ab, abortp)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t acc_base = tmem_base + ab * (uint32_t)(Cfg::NACC * Cfg::ACC_COLS);
+                const uint32_t acc_base = tmem_base + ab * (uint32_t)(NACC * Cfg::ACC_COLS);
                 for (int i = 0; i < nk; i++) {
-                    const uint32_t ready = MODE == 0 ? smem_u32(&bar_full[s]) : smem_u32(&bar_conv[s]);
-                    if (!known_ready && !mbar_wait(ready, ph, p.err, 0x200u + s, abortp)) { ok = false; break; }
+                    if (!known_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, p.err, 0x200u + s, abortp)) { ok = false; break; }
                     tc_fence_after();
                     {
                         const int s1 = (s + 1 == STAGES) ? 0 : s + 1;
                         const uint32_t ph1 = (s + 1 == STAGES) ? (ph ^ 1u) : ph;
-                        known_ready = mbar_test(MODE == 0 ? smem_u32(&bar_full[s1]) : smem_u32(&bar_conv[s1]), ph1);
+                        known_ready = mbar_test(smem_u32(&bar_full[s1]), ph1);
                     }
                     const uint64_t soff = (uint64_t)(((uint32_t)s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
 #pragma unroll
                     for (int ks = 0; ks < BK / 8; ks++) {
                         const uint64_t da = da0 + soff + (uint64_t)((ks * kstep_a) >> 4);
                         const uint64_t db = db0 + soff + (uint64_t)((ks * kstep_b) >> 4);
-                        if (MODE == 2) {
-                            // accumulator (ks % NACC); small cross terms first, then the main product
-                            const uint32_t acc = acc_base + (uint32_t)((ks % Cfg::NACC) * Cfg::ACC_COLS);
-                            const bool first = (i == 0) && (ks < Cfg::NACC);
-                            const uint64_t da_lo = da + (uint64_t)(Cfg::OPER_BYTES >> 4);
-                            const uint64_t db_lo = db + (uint64_t)(Cfg::OPER_BYTES >> 4);
-                            umma_tf32(acc, da_lo, db, idesc, first ? 0u : 1u);
-                            umma_tf32(acc, da, db_lo, idesc, 1u);
-                            umma_tf32(acc, da, db, idesc, 1u);
-                        } else {
-                            umma_tf32(acc_base, da, db, idesc, (uint32_t)((i | ks) != 0));
-                        }
+                        umma_tf32(acc_base + (uint32_t)((ks % NACC) * Cfg::ACC_COLS), da, db, idesc, (uint32_t)(i != 0 || ks >= NACC));
                     }
                     umma_commit(smem_u32(&bar_empty[s]));
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
@@ -398,12 +401,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             }
         }
     } else if (warp < 6) {
-        // ------------------------------ converter + epilogue warps ------------------------------
-        const int te = threadIdx.x - 64;  // 0..127
+        // ------------------------------ epilogue warps ------------------------------
         const int q = warp & 3;           // TMEM lane quadrant this warp may read
         const int r = q * 32 + lane;
-        int s = 0;
-        uint32_t ph = 0, tile_iter = 0;
+        uint32_t tile_iter = 0;
         bool ok = true;
         // CONVT output statistics: one running pair per channel tile, written once per CTA (see convh_kernel)
         double ssum = 0.0, ssq = 0.0;
@@ -415,12 +416,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                     sd[0] = 0.0; sd[1] = 0.0;
                 }
         for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, tile_iter++) {
-            const int n_tile = t % p.tiles_n, r_ = t / p.tiles_n, m_tile = r_ % p.tiles_m, z = r_ / p.tiles_m;
-            const int kt_begin = z * p.k_tiles_per_split;
-            int kt_end = kt_begin + p.k_tiles_per_split;
-            if (kt_end > p.num_k_tiles) kt_end = p.num_k_tiles;
-            const int nk = kt_end - kt_begin;
-            const int m0 = m_tile * BM, n0 = n_tile * BN;
+            const Tile T = tile_of(p, t);
+            const int m0 = T.m0, n0 = T.n_tile * BN;
             if (p.kind == KIND_CONVT && p.stat && m0 != stat_m0) {
                 if (stat_m0 >= 0 && stat_m0 + r < p.M) {
                     double* sd = p.stat + ((size_t)blockIdx.x * p.M + stat_m0 + r) * 2;
@@ -428,96 +425,69 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 }
                 ssum = 0.0; ssq = 0.0; stat_m0 = m0;
             }
-            if (MODE != 0) {
-                constexpr int NV = Cfg::OPER_BYTES / 16;
-                for (int i = 0; i < nk && ok; i++) {
-                    if (!mbar_wait(smem_u32(&bar_full[s]), ph, p.err, 0x300u + s, abortp)) { ok = false; break; }
-                    float4* buf = reinterpret_cast<float4*>(tiles_generic + (size_t)s * Cfg::STAGE_BYTES);
-                    float4* lo = reinterpret_cast<float4*>(tiles_generic + (size_t)s * Cfg::STAGE_BYTES + Cfg::OPER_BYTES);
-                    for (int j = te; j < NV; j += 128) {
-                        float4 v = buf[j];
-                        float4 h = make_float4(ncc::round_tf32(v.x), ncc::round_tf32(v.y), ncc::round_tf32(v.z), ncc::round_tf32(v.w));
-                        buf[j] = h;
-                        if (MODE == 2)
-                            lo[j] = make_float4(ncc::round_tf32(v.x - h.x), ncc::round_tf32(v.y - h.y),
-                                                ncc::round_tf32(v.z - h.z), ncc::round_tf32(v.w - h.w));
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive(smem_u32(&bar_conv[s]));
-                    if (++s == STAGES) { s = 0; ph ^= 1u; }
-                }
-            }
             const uint32_t ab = tile_iter % NBUF;
-            if (ok) ok = mbar_wait(smem_u32(&bar_acc_full[ab]), (tile_iter / NBUF) & 1u, p.err, 0x400u + ab, abortp);
+            ok = mbar_wait(smem_u32(&bar_acc_full[ab]), (tile_iter / NBUF) & 1u, p.err, 0x400u + ab, abortp);
             // all 32 lanes of a warp must agree before the aligned tcgen05.ld
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t acc_base = tmem_base + ab * (uint32_t)(Cfg::NACC * Cfg::ACC_COLS);
+            const uint32_t acc_base = tmem_base + ab * (uint32_t)(NACC * Cfg::ACC_COLS) + ((uint32_t)(q * 32) << 16);
+            // 32 accumulator columns of this warp's rows; after the last chunk the buffer may be overwritten by the tile after next
+            auto read_chunk = [&](int c0, bool last, uint32_t (&v)[32]) {
+                tmem_ld32(acc_base + (uint32_t)c0, v);
+                tmem_ld_wait();
+                if (NACC > 1) {
+#pragma unroll 1
+                    for (int a = 1; a < NACC; a++) {
+                        uint32_t u[32];
+                        tmem_ld32(acc_base + (uint32_t)(a * Cfg::ACC_COLS + c0), u);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+                    }
+                }
+                if (last) {
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&bar_acc_empty[ab]));
+                }
+            };
             if (p.kind == KIND_CONVT) {
                 // lane = output channel, column = pixel of the box; channels-last store: for one column the
                 // 32 lanes of a warp write 32 consecutive floats
+                const ConvClass& c = p.cls[T.cls];
                 const int co = m0 + r;
                 const bool co_ok = co < p.M;
                 const float bv = (co_ok && p.bias) ? p.bias[co] : 0.f;
-                const int tw = n_tile % p.tiles_w, tt = n_tile / p.tiles_w;
-                const int pw0 = tw * p.bw, ph0 = (tt % p.tiles_h) * p.bh, pn0 = (tt / p.tiles_h) * p.bn;
+                const int tw = T.px % c.tiles_w, tt = T.px / c.tiles_w;
+                const int pw0 = tw * p.bw, ph0 = (tt % c.tiles_h) * p.bh, pn0 = (tt / c.tiles_h) * p.bn;
+                const bool none = T.kt_end == T.kt_begin;   // a residue class no tap reaches: zeros
+                const int wstep = p.os * (int)p.ldd;        // between the class's neighbouring pixels of a row
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 32) {
                     float fs = 0.f, fq = 0.f;  // output statistics over the pixels of this chunk that exist
                     uint32_t v[32];
-                    tmem_ld32(acc_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-                    tmem_ld_wait();
-                    if (Cfg::NACC > 1) {
-#pragma unroll 1
-                        for (int a = 1; a < Cfg::NACC; a++) {
-                            uint32_t u[32];
-                            tmem_ld32(acc_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * Cfg::ACC_COLS + c0), u);
-                            tmem_ld_wait();
+                    read_chunk(c0, c0 + 32 >= BN, v);
+                    if (none)
 #pragma unroll
-                            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
-                        }
-                    }
-                    if (c0 + 32 >= BN) {
-                        tc_fence_before();
-                        mbar_arrive(smem_u32(&bar_acc_empty[ab]));
-                    }
-                    // the 32 columns of a chunk are runs of consecutive w inside one image row: the 64-bit
-                    // address is formed once per run, each store then adds a small constant multiple of ldd
-                    const int ldd = (int)p.ldd;
-                    if (p.bw >= 32) {
-                        const int w = pw0 + (c0 & (p.bw - 1));
-                        const int h = ph0 + ((c0 >> p.lbw) & (p.bh - 1));
-                        const int n = pn0 + (c0 >> (p.lbw + p.lbh));
-                        if (co_ok && h < p.Ho && n < p.Nimg) {
-                            float* dst = p.D + (((long long)n * p.Ho + h) * p.Wo + w) * p.ldd + co;
-                            const int lim = p.Wo - w;  // columns j < lim are inside the image
+                        for (int j = 0; j < 32; j++) v[j] = 0u;
+                    // the 32 columns of a chunk are runs of consecutive w inside one image row (a box is at least 8 wide): the
+                    // 64-bit address is formed once per run, each store then adds a small constant multiple of the step
 #pragma unroll
-                            for (int j = 0; j < 32; j++)
+                    for (int j0 = 0; j0 < 32; j0 += 8) {
+                        const int pj = c0 + j0;
+                        const int w = pw0 + (pj & (p.bw - 1));
+                        const int h = ph0 + ((pj >> p.lbw) & (p.bh - 1));
+                        const int n = pn0 + (pj >> (p.lbw + p.lbh));
+                        if (co_ok && h < c.Ho && n < p.Nimg) {
+                            float* dst = p.D + (((long long)n * p.Hout + c.oh0 + p.os * h) * p.Wout + c.ow0 + p.os * w) * p.ldd + co;
+                            const int lim = c.Wo - w;  // columns j < lim are inside the image
+#pragma unroll
+                            for (int j = 0; j < 8; j++)
                                 if (j < lim) {
-                                    const float o = __uint_as_float(v[j]) + bv;
-                                    dst[j * ldd] = o;
+                                    const float o = __uint_as_float(v[j0 + j]) + bv;
+                                    dst[j * wstep] = o;
                                     if (p.stat) { fs += o; fq = fmaf(o, o, fq); }
                                 }
-                        }
-                    } else {
-#pragma unroll
-                        for (int j0 = 0; j0 < 32; j0 += 8) {  // bw is 8 or 16: runs of 8 never cross a row
-                            const int pj = c0 + j0;
-                            const int w = pw0 + (pj & (p.bw - 1));
-                            const int h = ph0 + ((pj >> p.lbw) & (p.bh - 1));
-                            const int n = pn0 + (pj >> (p.lbw + p.lbh));
-                            if (co_ok && h < p.Ho && n < p.Nimg) {
-                                float* dst = p.D + (((long long)n * p.Ho + h) * p.Wo + w) * p.ldd + co;
-                                const int lim = p.Wo - w;
-#pragma unroll
-                                for (int j = 0; j < 8; j++)
-                                    if (j < lim) {
-                                        const float o = __uint_as_float(v[j0 + j]) + bv;
-                                        dst[j * ldd] = o;
-                                        if (p.stat) { fs += o; fq = fmaf(o, o, fq); }
-                                    }
-                            }
                         }
                     }
                     ssum += (double)fs;
@@ -528,77 +498,66 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             // where does this row go?
             long long row_off = -1;
             if (p.kind == KIND_CONV) {
-                const int tw = m_tile % p.tiles_w, tt = m_tile / p.tiles_w;
+                const int m_tile = m0 / BM, tw = m_tile % p.tiles_w, tt = m_tile / p.tiles_w;
                 const int cw0 = tw * p.bw, ch0 = (tt % p.tiles_h) * p.bh, cn0 = (tt / p.tiles_h) * p.bn;
                 const int iw = r % p.bw, t2 = r / p.bw, ih = t2 % p.bh, in_ = t2 / p.bh;
                 const int w = cw0 + iw, h = ch0 + ih, n = cn0 + in_;
                 if (w < p.Wo && h < p.Ho && n < p.Nimg) row_off = (((long long)n * p.Ho + h) * p.Wo + w) * p.ldd;
             } else {
                 const int m = m0 + r;
-                if (m < p.M) row_off = p.partial ? ((long long)z * p.M + m) * p.N : (long long)m * p.ldd;
+                if (m < p.M) row_off = p.partial ? ((long long)T.z * p.M + m) * p.N : (long long)m * p.ldd;
             }
             float* base = p.partial ? p.partial : p.D;
             const bool vec_ok = ((reinterpret_cast<uintptr_t>(base) & 15u) == 0) &&
                                 (((p.partial ? (long long)p.N : p.ldd) & 3) == 0);
+            // A thread holds 32 columns of ONE row, and storing them as they are would make every store instruction touch 32
+            // different lines: the block is turned through shared memory so that eight lanes store one row's 128 bytes
+            // (4096 x 4096 outputs, K = 1024: 87 -> MEASURED us).
+            float (*blk)[36] = turn[q];
+            const float alpha = p.partial ? 1.f : p.alpha, beta = p.partial ? 0.f : p.beta;
+            const float* biasv = p.partial ? nullptr : p.bias;
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 if (n0 + c0 >= p.N) break;  // uniform across the CTA
                 uint32_t v[32];
-                tmem_ld32(acc_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-                tmem_ld_wait();
-                if (Cfg::NACC > 1) {
-#pragma unroll 1
-                    for (int a = 1; a < Cfg::NACC; a++) {
-                        uint32_t u[32];
-                        tmem_ld32(acc_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * Cfg::ACC_COLS + c0), u);
-                        tmem_ld_wait();
+                read_chunk(c0, c0 + 32 >= BN || n0 + c0 + 32 >= p.N, v);
+                __syncwarp();
 #pragma unroll
-                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
-                    }
-                }
-                if (c0 + 32 >= BN || n0 + c0 + 32 >= p.N) {
-                    // last chunk read: the accumulator buffer may be overwritten by the tile after next
-                    tc_fence_before();
-                    mbar_arrive(smem_u32(&bar_acc_empty[ab]));
-                }
-                if (row_off < 0) continue;
-                float* dst = base + row_off + n0 + c0;
+                for (int j = 0; j < 32; j += 4)
+                    *reinterpret_cast<float4*>(&blk[lane][j]) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                                            __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                __syncwarp();
                 const int ncols = (p.N - (n0 + c0)) < 32 ? (p.N - (n0 + c0)) : 32;
-                if (p.partial) {
-                    if (vec_ok && ncols == 32) {
+                if (vec_ok && ncols == 32) {
+                    const int cl = (lane & 7) * 4;
+                    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (biasv) { const float* bp = biasv + n0 + c0 + cl; b4 = make_float4(bp[0], bp[1], bp[2], bp[3]); }
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                              __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (j < ncols) dst[j] = __uint_as_float(v[j]);
+                    for (int it = 0; it < 8; it++) {
+                        const int row = it * 4 + (lane >> 3);
+                        const long long ro = __shfl_sync(0xffffffffu, row_off, row);
+                        float4 o = *reinterpret_cast<const float4*>(&blk[row][cl]);
+                        if (ro < 0) continue;
+                        float4* dst = reinterpret_cast<float4*>(base + ro + n0 + c0 + cl);
+                        o.x *= alpha; o.y *= alpha; o.z *= alpha; o.w *= alpha;
+                        if (beta != 0.f) {
+                            const float4 old = *dst;
+                            o.x += beta * old.x; o.y += beta * old.y; o.z += beta * old.z; o.w += beta * old.w;
+                        }
+                        if (biasv) { o.x += b4.x; o.y += b4.y; o.z += b4.z; o.w += b4.w; }
+                        *dst = o;
                     }
                 } else {
-                    const float* bias = p.bias ? p.bias + n0 + c0 : nullptr;
-                    if (vec_ok && ncols == 32) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4) {
-                            float4 o = make_float4(p.alpha * __uint_as_float(v[j]), p.alpha * __uint_as_float(v[j + 1]),
-                                                   p.alpha * __uint_as_float(v[j + 2]), p.alpha * __uint_as_float(v[j + 3]));
-                            if (p.beta != 0.f) {
-                                float4 old = *reinterpret_cast<const float4*>(dst + j);
-                                o.x += p.beta * old.x; o.y += p.beta * old.y; o.z += p.beta * old.z; o.w += p.beta * old.w;
-                            }
-                            if (bias) { o.x += bias[j]; o.y += bias[j + 1]; o.z += bias[j + 2]; o.w += bias[j + 3]; }
-                            *reinterpret_cast<float4*>(dst + j) = o;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            if (j < ncols) {
-                                float o = p.alpha * __uint_as_float(v[j]);
-                                if (p.beta != 0.f) o += p.beta * dst[j];
-                                if (bias) o += bias[j];
-                                dst[j] = o;
-                            }
-                        }
+                    const float b1 = (biasv && lane < ncols) ? biasv[n0 + c0 + lane] : 0.f;
+#pragma unroll 4
+                    for (int row = 0; row < 32; row++) {
+                        const long long ro = __shfl_sync(0xffffffffu, row_off, row);
+                        if (ro < 0 || lane >= ncols) continue;
+                        float* dst = base + ro + n0 + c0 + lane;
+                        float o = alpha * blk[row][lane];
+                        if (beta != 0.f) o += beta * *dst;
+                        if (biasv) o += b1;
+                        *dst = o;
                     }
                 }
             }
@@ -626,8 +585,59 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 }
 
 // ------------------------------------------------------------------------------------------
-// Second stages and weight packing
+// Operand preparation, second stages and weight packing
 // ------------------------------------------------------------------------------------------
+// dst plane 0 = src rounded to nearest TF32; plane 1 (when there are two) = the rounded remainder.  Rows of ld_dst floats (a multiple
+// of four, 16-byte aligned), zeros where dst is larger than src: also turns operands TMA cannot describe (odd leading dimensions,
+// misaligned bases) into ones it can.
+template <bool VEC>
+__global__ void __launch_bounds__(256) split_operand_kernel(float* __restrict__ dst, const float* __restrict__ src, size_t rows, int cols,
+                                                            size_t ld_src, size_t rows_dst, int ld_dst, int planes) {
+    ncc::pdl_wait();
+    const int q4 = ld_dst >> 2;
+    const size_t total = rows_dst * q4, plane = rows_dst * (size_t)ld_dst, stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const size_t r = i / q4;
+        const int c = (int)(i - r * q4) * 4;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (r < rows) {
+            const float* s = src + r * ld_src + c;
+            if (VEC && c + 4 <= cols) {
+                const float4 t = *reinterpret_cast<const float4*>(s);
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) if (c + e < cols) v[e] = s[e];
+            }
+        }
+        float h[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) h[e] = ncc::round_tf32(v[e]);
+        *reinterpret_cast<float4*>(dst + r * ld_dst + c) = make_float4(h[0], h[1], h[2], h[3]);
+        if (planes == 2)
+            *reinterpret_cast<float4*>(dst + plane + r * ld_dst + c) =
+                make_float4(ncc::round_tf32(v[0] - h[0]), ncc::round_tf32(v[1] - h[1]), ncc::round_tf32(v[2] - h[2]), ncc::round_tf32(v[3] - h[3]));
+    }
+}
+// scratch copy of an operand; rows_dst >= rows.  nullptr: no memory (status set)
+static float* split_operand(int slot, const float* src, size_t rows, int cols, size_t ld_src, size_t rows_dst, int ld_dst, int planes,
+                            cudaStream_t st) {
+    float* dst = (float*)ncc::scratch(slot, sizeof(float) * rows_dst * ld_dst * planes, st);
+    if (!dst) return nullptr;
+    const bool vec = ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+    const int grid = ncc::grid_for((long long)(rows_dst * (ld_dst / 4)), 256);
+    if (vec) ncc::launch(split_operand_kernel<true>, grid, 256, 0, st, dst, src, rows, cols, ld_src, rows_dst, ld_dst, planes);
+    else ncc::launch(split_operand_kernel<false>, grid, 256, 0, st, dst, src, rows, cols, ld_src, rows_dst, ld_dst, planes);
+    NCC_COUNT_LAUNCH();
+    return ncc::launch_status("split_operand") == NC_CUDA_OK ? dst : nullptr;
+}
+constexpr int kSlotA = 10, kSlotB = 11;
+int mode_planes(int mode) { return mode == NC_CUDA_MATH_3XTF32 ? 2 : 1; }
+// a dense channels-last activation as the math mode wants it: itself (TF32), rounded (RNA), hi and lo planes N images apart (3xTF32)
+static const float* split_pixels(int slot, const float* x, size_t pixels, int C, int mode, cudaStream_t st) {
+    return mode == NC_CUDA_MATH_TF32 ? x : split_operand(slot, x, pixels, C, (size_t)C, pixels, C, mode_planes(mode), st);
+}
+
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ D, long long ldd, const float* __restrict__ partial,
                                                             int splits, int M, int N, const float* __restrict__ bias,
                                                             float alpha, float beta) {
@@ -653,15 +663,16 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
     }
 }
 
-// partial[z][co][(kh*kW+kw)*Cin + ci]  ->  dW[co][ci][kh][kw].  Threads walk the SOURCE order (coalesced reads of every split;
-// walking the destination order reads with a stride of Cin floats, eight times the sectors), eight splits are requested
-// before the first one is added, and only the single write per element is scattered.
+// partial[z][co][(kh*kW+kw)*Cp + ci]  ->  dW[co][ci][kh][kw], Cp = Cin padded to whole 32-channel chunks.  Threads walk the SOURCE
+// order (coalesced reads of every split; walking the destination order reads with a stride of Cin floats, eight times the sectors),
+// eight splits are requested before the first one is added, and only the single write per element is scattered.
 __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, const float* __restrict__ partial, int splits,
-                                                        int Cout, int Cin, int kH, int kW) {
+                                                        int Cout, int Cin, int Cp, int T) {
     ncc::pdl_wait();
-    const int T = kH * kW;
-    const size_t total = (size_t)Cout * Cin * T, stride = (size_t)gridDim.x * blockDim.x;
+    const size_t total = (size_t)Cout * Cp * T, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t src = (size_t)blockIdx.x * blockDim.x + threadIdx.x; src < total; src += stride) {
+        const int ci = (int)(src % Cp);
+        if (ci >= Cin) continue;
         double acc = 0.0;
         int z = 0;
         for (; z + 8 <= splits; z += 8) {
@@ -672,39 +683,38 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, 
             for (int k = 0; k < 8; k++) acc += (double)v[k];
         }
         for (; z < splits; z++) acc += (double)partial[(size_t)z * total + src];
-        const int ci = (int)(src % Cin);
-        const size_t r = src / Cin;
+        const size_t r = src / Cp;
         const int tap = (int)(r % T);
         const size_t co = r / T;
         dW[(co * Cin + ci) * T + tap] = (float)acc;
     }
 }
 
+// dst[plane][tap][out][in], `in` the channels of the reduction; tap t takes filter position at[t].  DX: out = ci, in = co.
+struct TapOrder { unsigned char at[64]; };
 template <bool DX>
 __global__ void __launch_bounds__(256) pack_weights_kernel(float* __restrict__ wp, const float* __restrict__ w, int Cout, int Cin,
-                                                           int kH, int kW, int round) {
+                                                           int T, const __grid_constant__ TapOrder order, int round, int planes) {
     ncc::pdl_wait();
-    const size_t total = (size_t)Cout * Cin * kH * kW, stride = (size_t)gridDim.x * blockDim.x;
+    const size_t total = (size_t)Cout * Cin * T, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         size_t r = i;
-        int kh, kw, co, ci;
-        if (!DX) {  // dst (kh, kw, co, ci)
-            ci = r % Cin; r /= Cin; co = r % Cout; r /= Cout; kw = r % kW; kh = (int)(r / kW);
-        } else {    // dst (kh', kw', ci, co), source taps flipped
-            co = r % Cout; r /= Cout; ci = r % Cin; r /= Cin; kw = r % kW; kh = (int)(r / kW);
-            kh = kH - 1 - kh; kw = kW - 1 - kw;
-        }
-        float v = w[(((size_t)co * Cin + ci) * kH + kh) * kW + kw];
-        wp[i] = round ? ncc::round_tf32(v) : v;
+        int co, ci;
+        if (!DX) { ci = r % Cin; r /= Cin; co = r % Cout; r /= Cout; }
+        else { co = r % Cout; r /= Cout; ci = r % Cin; r /= Cin; }
+        const float v = w[((size_t)co * Cin + ci) * T + order.at[r]];
+        const float h = round ? ncc::round_tf32(v) : v;
+        wp[i] = h;
+        if (planes == 2) wp[total + i] = ncc::round_tf32(v - h);
     }
 }
 
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-template <int BN, bool A_MN, bool B_MN, int MODE>
+template <int BN, bool A_MN, bool B_MN, int NACC>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p_in, dim3 tiles, cudaStream_t st) {
-    using Cfg = TileCfg<BN, MODE>;
+    using Cfg = TileCfg<BN, NACC>;
     TcParams p = p_in;
     p.tiles_n = (int)tiles.x; p.tiles_m = (int)tiles.y; p.splits = (int)tiles.z;
     p.stages = Cfg::STAGES;
@@ -712,7 +722,7 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcPara
     const int sms = ncc::sm_count();
     dim3 grid((unsigned)(total < sms ? total : sms), 1, 1);
     static bool attr_set = false;
-    auto kern = tc_kernel<BN, A_MN, B_MN, MODE>;
+    auto kern = tc_kernel<BN, A_MN, B_MN, NACC>;
     if (!attr_set) {
         NCC_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_set = true;
@@ -725,28 +735,19 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcPara
     return ncc::launch_status("tc_kernel");
 }
 
-template <int BN, bool A_MN, bool B_MN>
-static int launch_mode(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p, dim3 grid, cudaStream_t st) {
-    switch (mode) {
-        case NC_CUDA_MATH_TF32: return launch_one<BN, A_MN, B_MN, 0>(ta, tb, p, grid, st);
-        case NC_CUDA_MATH_TF32_RNA: return launch_one<BN, A_MN, B_MN, 1>(ta, tb, p, grid, st);
-        case NC_CUDA_MATH_3XTF32: return launch_one<BN, A_MN, B_MN, 2>(ta, tb, p, grid, st);
-    }
-    return ncc::set_status(NC_CUDA_ERR_ARG, "tc: unknown math mode %d", mode);
-}
-
 template <bool A_MN, bool B_MN>
-static int launch_bn(int bn, int mode, const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p, dim3 grid, cudaStream_t st) {
+static int launch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p, dim3 grid, cudaStream_t st) {
+    const bool two = p.kind == KIND_GEMM && p.passes == 3;   // two accumulators
     switch (bn) {
-        case 64: return launch_mode<64, A_MN, B_MN>(mode, ta, tb, p, grid, st);
-        case 128: return launch_mode<128, A_MN, B_MN>(mode, ta, tb, p, grid, st);
-        case 256: return launch_mode<256, A_MN, B_MN>(mode, ta, tb, p, grid, st);
+        case 64: return two ? launch_one<64, A_MN, B_MN, 2>(ta, tb, p, grid, st) : launch_one<64, A_MN, B_MN, 1>(ta, tb, p, grid, st);
+        case 128: return two ? launch_one<128, A_MN, B_MN, 2>(ta, tb, p, grid, st) : launch_one<128, A_MN, B_MN, 1>(ta, tb, p, grid, st);
+        case 256: return launch_one<256, A_MN, B_MN, 1>(ta, tb, p, grid, st);
     }
     return ncc::set_status(NC_CUDA_ERR_ARG, "tc: unsupported tile width %d", bn);
 }
 
-// 3xTF32 prefers 128-column tiles: four accumulators fit in tensor memory instead of two.
-static int pick_bn(int N, int mode = 0) { return N <= 64 ? 64 : ((N <= 128 || mode == NC_CUDA_MATH_3XTF32) ? 128 : 256); }
+// two accumulators of a 3xTF32 product (and their double buffering) fit in tensor memory for up to 128 columns
+static int pick_bn(int N, bool two_acc = false) { return N <= 64 ? 64 : ((N <= 128 || two_acc) ? 128 : 256); }
 
 // splits over the reduction so that about one wave of CTAs exists; each split keeps >= 4 tiles
 static void pick_splits(int tiles, int nk, int* splits, int* kps) {
@@ -762,27 +763,46 @@ static void pick_splits(int tiles, int nk, int* splits, int* kps) {
     *splits = (nk + per - 1) / per;
 }
 
+// Rows beyond M inside the 128-row tile are zero-filled by TMA and never stored; small products stay on CUDA cores.  Operands whose
+// rows are no whole 16-byte pieces cost a copy each first: from 2^24 multiply-adds on.
+bool gemm_eligible(int M, int N, int K, bool aligned) {
+    return M >= 32 && N >= 16 && K >= 32 && (long long)M * N * K >= (aligned ? 1ll << 22 : 1ll << 24);
+}
+
 int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N, int K,
          const float* bias, float alpha, float beta, int mode, cudaStream_t st) {
-    // rows beyond M inside the 128-row tile are zero-filled by TMA and never stored; tiny problems stay on the SIMT kernel
-    if (M < 32 || N < 16 || K < 32 || (long long)M * N * K < (1ll << 22)) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((lda & 3) || (ldb & 3)) return NC_CUDA_ERR_UNSUPPORTED;
-    const int bn = pick_bn(N, mode);
+    const bool a_ok = !(lda & 3) && !(reinterpret_cast<uintptr_t>(A) & 15u), b_ok = !(ldb & 3) && !(reinterpret_cast<uintptr_t>(B) & 15u);
+    if (!gemm_eligible(M, N, K, a_ok && b_ok)) return NC_CUDA_ERR_UNSUPPORTED;
+    const int planes = mode_planes(mode), k_rows = planes == 2 ? (K + BK - 1) / BK * BK : K;
+    // the reduction ends at K: along a row the tensor map's extent says so, along the rows of a split MN-major operand zeros do
+    auto prepare = [&](int slot, const float*& X, int& ld, bool mn, int outer, bool ok) {
+        if (mode == NC_CUDA_MATH_TF32 && ok) return true;
+        const int rows = mn ? K : outer, cols = mn ? outer : K, ldp = (cols + 3) & ~3;
+        const float* c = split_operand(slot, X, (size_t)rows, cols, (size_t)ld, (size_t)(mn ? k_rows : outer), ldp, planes, st);
+        if (!c) return false;
+        X = c; ld = ldp;
+        return true;
+    };
+    if (!prepare(kSlotA, A, lda, a_mn, M, a_ok) || !prepare(kSlotB, B, ldb, b_mn, N, b_ok)) return NC_CUDA_ERR_RUNTIME;
+    const int bn = pick_bn(N, planes == 2);
     CUtensorMap ta, tb;
     {
         unsigned long long dims[2], str[1];
         unsigned box[2];
-        if (!a_mn) { dims[0] = K; dims[1] = M; str[0] = lda; box[0] = 32; box[1] = 128; }
-        else       { dims[0] = M; dims[1] = K; str[0] = lda; box[0] = 32; box[1] = 32; }
+        if (!a_mn) { dims[0] = K; dims[1] = (unsigned long long)M * planes; str[0] = lda; box[0] = 32; box[1] = 128; }
+        else       { dims[0] = M; dims[1] = (unsigned long long)k_rows * planes; str[0] = lda; box[0] = 32; box[1] = 32; }
         if (!make_map(&ta, A, 2, dims, str, box, a_mn)) return NC_CUDA_ERR_UNSUPPORTED;
-        if (!b_mn) { dims[0] = K; dims[1] = N; str[0] = ldb; box[0] = 32; box[1] = (unsigned)bn; }
-        else       { dims[0] = N; dims[1] = K; str[0] = ldb; box[0] = 32; box[1] = 32; }
+        if (!b_mn) { dims[0] = K; dims[1] = (unsigned long long)N * planes; str[0] = ldb; box[0] = 32; box[1] = (unsigned)bn; }
+        else       { dims[0] = N; dims[1] = (unsigned long long)k_rows * planes; str[0] = ldb; box[0] = 32; box[1] = 32; }
         if (!make_map(&tb, B, 2, dims, str, box, b_mn)) return NC_CUDA_ERR_UNSUPPORTED;
     }
     TcParams p = {};
     p.kind = KIND_GEMM;
     p.M = M; p.N = N;
-    p.num_k_tiles = (K + BK - 1) / BK;
+    p.passes = planes == 2 ? 3 : 1;
+    p.pass_tiles = (K + BK - 1) / BK;
+    p.a_plane = a_mn ? k_rows : M; p.b_plane = b_mn ? k_rows : N;
+    p.num_k_tiles = p.pass_tiles * p.passes;
     p.D = D; p.ldd = ldd; p.bias = bias; p.alpha = alpha; p.beta = beta;
     p.err = ncc::device_error_word();
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
@@ -796,10 +816,10 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
     dim3 grid(tiles_n, tiles_m, splits);
     p.flops = 2.0 * M * (double)N * K;
     int rc;
-    if (!a_mn && !b_mn) rc = launch_bn<false, false>(bn, mode, ta, tb, p, grid, st);
-    else if (!a_mn && b_mn) rc = launch_bn<false, true>(bn, mode, ta, tb, p, grid, st);
-    else if (a_mn && !b_mn) rc = launch_bn<true, false>(bn, mode, ta, tb, p, grid, st);
-    else rc = launch_bn<true, true>(bn, mode, ta, tb, p, grid, st);
+    if (!a_mn && !b_mn) rc = launch_bn<false, false>(bn, ta, tb, p, grid, st);
+    else if (!a_mn && b_mn) rc = launch_bn<false, true>(bn, ta, tb, p, grid, st);
+    else if (a_mn && !b_mn) rc = launch_bn<true, false>(bn, ta, tb, p, grid, st);
+    else rc = launch_bn<true, true>(bn, ta, tb, p, grid, st);
     if (rc) return rc;
     if (splits > 1) {
         ncc::launch(splitk_reduce_kernel, ncc::grid_for((long long)M * N, 256), 256, 0, st, D, ldd, p.partial, splits, M, N, bias, alpha, beta);
@@ -810,12 +830,12 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
 }
 
 // Pixel box (bw, bh, bn) with bw*bh*bn == pixels that wastes the fewest rows for this image size.
-static void pick_box(int pixels, int Wd, int Hd, int Nd, int* bw, int* bh, int* bn, int min_w = 1) {
+static void pick_box(int pixels, int Wd, int Hd, int Nd, int* bw, int* bh, int* bn, int min_w = 1, int max_side = 256, bool whole_images = false) {
     long long best = -1;
     for (int w = min_w; w <= pixels; w *= 2)
         for (int h = 1; w * h <= pixels; h *= 2) {
             int n = pixels / (w * h);
-            if (w * h * n != pixels || w > 256 || h > 256 || n > 256) continue;
+            if (w * h * n != pixels || w > max_side || h > max_side || n > 256 || (whole_images && Nd % n)) continue;
             long long cover = (long long)((Wd + w - 1) / w) * w * ((Hd + h - 1) / h) * h * ((Nd + n - 1) / n) * n;
             // prefer less waste, then wider rows (longer contiguous runs), then fewer images per box
             if (best < 0 || cover < best || (cover == best && (w > *bw || (w == *bw && n < *bn)))) {
@@ -824,65 +844,93 @@ static void pick_box(int pixels, int Wd, int Hd, int Nd, int* bw, int* bh, int* 
         }
 }
 
+bool conv_eligible(int Cin, int Cout, long long pixels) {
+    return !(Cin & 3) && !(Cout & 3) && Cin >= 16 && Cout >= 16 && pixels >= 128;
+}
+
+// CONVT launch: the given classes over x (N,H,W,Cin) with input pixel stride `stride`, into y (N,Hout,Wout,Cout) with output pixel
+// stride `os`.  xs: x as split_pixels made it.
+static int convt_launch(float* y, int Hout, int Wout, int os, const float* xs, const float* wpacked, long long wrows_total, const float* bias,
+                        int N, int H, int W, int Cin, int Cout, int stride, ConvClass* cls, int classes, int mode, bool want_stats,
+                        double flops, cudaStream_t st) {
+    const int planes = mode_planes(mode);
+    int mh = 0, mw = 0;
+    for (int i = 0; i < classes; i++) { mh = cls[i].Ho > mh ? cls[i].Ho : mh; mw = cls[i].Wo > mw ? cls[i].Wo : mw; }
+    int bw = 1, bh = 1, bnn = 1;
+    pick_box(256, mw, mh, N, &bw, &bh, &bnn, 8, 256 / stride);
+    CUtensorMap ta, tb;
+    unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)wrows_total * planes};
+    unsigned long long ws[1] = {(unsigned long long)Cin};
+    unsigned wb[2] = {32, 128};
+    if (!make_map(&ta, wpacked, 2, wd, ws, wb, false)) return NC_CUDA_ERR_UNSUPPORTED;
+    unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N * planes};
+    unsigned long long str[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
+    unsigned box[4] = {32, (unsigned)bw, (unsigned)bh, (unsigned)bnn};
+    if (!make_map(&tb, xs, 4, dims, str, box, false, stride)) return NC_CUDA_ERR_UNSUPPORTED;
+    TcParams p = {};
+    p.kind = KIND_CONVT;
+    p.M = Cout;
+    p.cchunks = (Cin + 31) / 32;
+    p.passes = planes == 2 ? 3 : 1;
+    p.a_plane = (int)wrows_total; p.b_plane = N;
+    p.D = y; p.ldd = Cout; p.bias = bias; p.alpha = 1.f; p.beta = 0.f;
+    p.bw = bw; p.bh = bh; p.bn = bnn;
+    for (p.lbw = 0; (1 << p.lbw) < bw; p.lbw++) {}
+    for (p.lbh = 0; (1 << p.lbh) < bh; p.lbh++) {}
+    p.Nimg = N;
+    p.stride = stride; p.wrows = Cout;
+    p.classes = classes; p.os = os; p.Hout = Hout; p.Wout = Wout;
+    p.err = ncc::device_error_word();
+    long long tiles_px = 0;
+    for (int i = 0; i < classes; i++) {
+        cls[i].tiles_w = (cls[i].Wo + bw - 1) / bw; cls[i].tiles_h = (cls[i].Ho + bh - 1) / bh;
+        cls[i].tile0 = (int)tiles_px;
+        tiles_px += (long long)cls[i].tiles_w * cls[i].tiles_h * ((N + bnn - 1) / bnn);
+        p.cls[i] = cls[i];
+    }
+    if (tiles_px > (1ll << 30)) return NC_CUDA_ERR_UNSUPPORTED;
+    p.N = 0x7fffffff;
+    p.pass_tiles = p.k_tiles_per_split = p.num_k_tiles = 1;   // per class, see tile_of
+    dim3 tiles((unsigned)tiles_px, (unsigned)((Cout + BM - 1) / BM), 1);
+    p.flops = flops;
+    // launch_one uses min(tiles, SMs) persistent CTAs: one statistics slab per CTA
+    const long long total_tiles = (long long)tiles.x * tiles.y;
+    const int n_ctas = (int)(total_tiles < ncc::sm_count() ? total_tiles : ncc::sm_count());
+    if (want_stats) p.stat = ncc::conv_stats_buffer((size_t)n_ctas, Cout, st);
+    const int rc = launch_one<256, false, false, 1>(ta, tb, p, tiles, st);
+    if (rc == NC_CUDA_OK && p.stat) ncc::conv_stats_publish(y, Cout, (long long)N * Hout * Wout, n_ctas, p.stat);
+    return rc;
+}
+
 int conv_nhwc(float* y, const float* x, const float* wpacked, const float* bias, int N, int H, int W, int Cin, int Cout,
               int kH, int kW, int pad, int mode, cudaStream_t st) {
     const int Ho = H + 2 * pad - kH + 1, Wo = W + 2 * pad - kW + 1;
     if (Ho <= 0 || Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((Cin & 3) || (Cout & 3) || Cin < 16 || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((long long)N * Ho * Wo < 128) return NC_CUDA_ERR_UNSUPPORTED;
+    if (!conv_eligible(Cin, Cout, (long long)N * Ho * Wo)) return NC_CUDA_ERR_UNSUPPORTED;
+    const float* xs = split_pixels(kSlotA, x, (size_t)N * H * W, Cin, mode, st);
+    if (!xs) return NC_CUDA_ERR_RUNTIME;
+    const int planes = mode_planes(mode);
     {
-        const int rc = conv_halo_nhwc(y, x, wpacked, bias, N, H, W, Cin, Cout, kH, kW, pad, mode, st);
+        const int rc = conv_halo_nhwc(y, xs, wpacked, bias, N, H, W, Cin, Cout, kH, kW, pad, planes, st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
+    const double flops = 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW;
     if ((long long)N * Ho * Wo >= 1024 && kH * kW * Cout >= 128) {
         // pixels on the N side (256 per tile), channels on the M side
-        int bw = 1, bh = 1, bnn = 1;
-        pick_box(256, Wo, Ho, N, &bw, &bh, &bnn, 8);
-        CUtensorMap ta, tb;
-        unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout};
-        unsigned long long ws[1] = {(unsigned long long)Cin};
-        unsigned wb[2] = {32, 128};
-        if (!make_map(&ta, wpacked, 2, wd, ws, wb, false)) return NC_CUDA_ERR_UNSUPPORTED;
-        unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N};
-        unsigned long long str[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
-        unsigned box[4] = {32, (unsigned)bw, (unsigned)bh, (unsigned)bnn};
-        if (!make_map(&tb, x, 4, dims, str, box, false)) return NC_CUDA_ERR_UNSUPPORTED;
-        TcParams p = {};
-        p.kind = KIND_CONVT;
-        p.M = Cout;
-        p.cchunks = (Cin + 31) / 32;
-        p.num_k_tiles = kH * kW * p.cchunks;
-        p.k_tiles_per_split = p.num_k_tiles;
-        p.D = y; p.ldd = Cout; p.bias = bias; p.alpha = 1.f; p.beta = 0.f;
-        p.bw = bw; p.bh = bh; p.bn = bnn;
-        for (p.lbw = 0; (1 << p.lbw) < bw; p.lbw++) {}
-        for (p.lbh = 0; (1 << p.lbh) < bh; p.lbh++) {}
-        p.tiles_w = (Wo + bw - 1) / bw; p.tiles_h = (Ho + bh - 1) / bh;
-        p.Ho = Ho; p.Wo = Wo; p.Nimg = N;
-        p.kW = kW; p.pad = pad; p.wrows = Cout;
-        p.err = ncc::device_error_word();
-        const long long tiles_px = (long long)p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
-        p.N = (int)(tiles_px * 256 < 0x7fffffffLL ? tiles_px * 256 : 0x7fffffff);
-        dim3 tiles((unsigned)tiles_px, (unsigned)((Cout + BM - 1) / BM), 1);
-        p.flops = 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW;
-        // launch_one uses min(tiles, SMs) persistent CTAs: one statistics slab per CTA
-        const long long total_tiles = (long long)tiles.x * tiles.y;
-        const int n_ctas = (int)(total_tiles < ncc::sm_count() ? total_tiles : ncc::sm_count());
-        if (ncc::conv_stats_wanted()) p.stat = ncc::conv_stats_buffer((size_t)n_ctas, Cout, st);
-        const int rc = launch_mode<256, false, false>(mode, ta, tb, p, tiles, st);
-        if (rc == NC_CUDA_OK && p.stat) ncc::conv_stats_publish(y, Cout, (long long)N * Ho * Wo, n_ctas, p.stat);
-        return rc;
+        ConvClass c = {};
+        c.kH = kH; c.kW = kW; c.pad_h = c.pad_w = pad; c.Ho = Ho; c.Wo = Wo;
+        return convt_launch(y, Ho, Wo, 1, xs, wpacked, (long long)kH * kW * Cout, bias, N, H, W, Cin, Cout, 1, &c, 1, mode, ncc::conv_stats_wanted(), flops, st);
     }
-    const int bn_cols = pick_bn(Cout, mode);
+    const int bn_cols = pick_bn(Cout);
     int bw = 1, bh = 1, bnn = 1;
     pick_box(128, Wo, Ho, N, &bw, &bh, &bnn);
     CUtensorMap ta, tb;
     {
-        unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N};
+        unsigned long long dims[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N * planes};
         unsigned long long str[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
         unsigned box[4] = {32, (unsigned)bw, (unsigned)bh, (unsigned)bnn};
-        if (!make_map(&ta, x, 4, dims, str, box, false)) return NC_CUDA_ERR_UNSUPPORTED;
-        unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout};
+        if (!make_map(&ta, xs, 4, dims, str, box, false)) return NC_CUDA_ERR_UNSUPPORTED;
+        unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout * planes};
         unsigned long long ws[1] = {(unsigned long long)Cin};
         unsigned wb[2] = {32, (unsigned)bn_cols};
         if (!make_map(&tb, wpacked, 2, wd, ws, wb, false)) return NC_CUDA_ERR_UNSUPPORTED;
@@ -891,7 +939,10 @@ int conv_nhwc(float* y, const float* x, const float* wpacked, const float* bias,
     p.kind = KIND_CONV;
     p.M = N * Ho * Wo; p.N = Cout;
     p.cchunks = (Cin + 31) / 32;
-    p.num_k_tiles = kH * kW * p.cchunks;
+    p.passes = planes == 2 ? 3 : 1;
+    p.pass_tiles = kH * kW * p.cchunks;
+    p.a_plane = N; p.b_plane = kH * kW * Cout;
+    p.num_k_tiles = p.pass_tiles * p.passes;
     p.k_tiles_per_split = p.num_k_tiles;
     p.D = y; p.ldd = Cout; p.bias = bias; p.alpha = 1.f; p.beta = 0.f;
     p.bw = bw; p.bh = bh; p.bn = bnn;
@@ -901,35 +952,89 @@ int conv_nhwc(float* y, const float* x, const float* wpacked, const float* bias,
     p.err = ncc::device_error_word();
     const long long tiles_m = (long long)p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
     dim3 grid((Cout + bn_cols - 1) / bn_cols, (unsigned)tiles_m, 1);
-    p.flops = 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW;
-    return launch_bn<false, false>(bn_cols, mode, ta, tb, p, grid, st);
+    p.flops = flops;
+    return launch_bn<false, false>(bn_cols, ta, tb, p, grid, st);
 }
 
-int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W, int Cin, int Cout, int kH, int kW, int pad,
+int conv_strided_nhwc(float* y, const float* x, const float* wpacked, const float* bias, int N, int H, int W, int Cin, int Cout,
+                      int kH, int kW, int stride, int pad, int mode, cudaStream_t st) {
+    const int Ho = (H + 2 * pad - kH) / stride + 1, Wo = (W + 2 * pad - kW) / stride + 1;
+    if (!conv_strided_eligible(Cin, Cout, (long long)N * Ho * Wo, kH, kW, stride)) return NC_CUDA_ERR_UNSUPPORTED;
+    const float* xs = split_pixels(kSlotA, x, (size_t)N * H * W, Cin, mode, st);
+    if (!xs) return NC_CUDA_ERR_RUNTIME;
+    ConvClass c = {};
+    c.kH = kH; c.kW = kW; c.pad_h = c.pad_w = pad; c.Ho = Ho; c.Wo = Wo;
+    return convt_launch(y, Ho, Wo, 1, xs, wpacked, (long long)kH * kW * Cout, bias, N, H, W, Cin, Cout, stride, &c, 1, mode,
+                        ncc::conv_stats_wanted(), 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW, st);
+}
+
+// Input coordinate h of residue class r is h = s * i + r; filter row kh reaches it from output row (h + pad - kh) / s, so with
+// kh0 = (r + pad) mod s only the taps kh0, kh0 + s, ... count, and output row = i + (r + pad - kh0) / s - t for the t-th of them.
+// Reversed, they are an ordinary stride-1 filter over dy with padding taps - 1 - (r + pad - kh0) / s.
+static void residue_axis(int r, int k, int s, int pad, int extent, int* kh0, int* taps, int* cpad, int* outs) {
+    *kh0 = (r + pad) % s;
+    *taps = *kh0 < k ? (k - *kh0 + s - 1) / s : 0;
+    *cpad = *taps - 1 - (r + pad - *kh0) / s;
+    *outs = r < extent ? (extent - r + s - 1) / s : 0;
+}
+int conv_dx_strided_nhwc(float* dx, const float* dy, const float* wpacked, int N, int H, int W, int Cin, int Cout, int kH, int kW,
+                         int stride, int pad, int mode, cudaStream_t st) {
+    const int Ho = (H + 2 * pad - kH) / stride + 1, Wo = (W + 2 * pad - kW) / stride + 1;
+    if (!conv_strided_eligible(Cout, Cin, (long long)N * H * W, kH, kW, stride)) return NC_CUDA_ERR_UNSUPPORTED;
+    const float* ds = split_pixels(kSlotA, dy, (size_t)N * Ho * Wo, Cout, mode, st);
+    if (!ds) return NC_CUDA_ERR_RUNTIME;
+    ConvClass cls[kMaxClasses] = {};
+    int n = 0, row = 0;
+    for (int rh = 0; rh < stride; rh++)
+        for (int rw = 0; rw < stride; rw++) {
+            ConvClass c = {};
+            int a, b;
+            residue_axis(rh, kH, stride, pad, H, &a, &c.kH, &c.pad_h, &c.Ho);
+            residue_axis(rw, kW, stride, pad, W, &b, &c.kW, &c.pad_w, &c.Wo);
+            c.oh0 = rh; c.ow0 = rw;
+            c.wrow0 = row * Cin;
+            row += c.kH * c.kW;
+            if (c.Ho > 0 && c.Wo > 0) cls[n++] = c;
+        }
+    return convt_launch(dx, H, W, stride, ds, wpacked, (long long)kH * kW * Cin, nullptr, N, Ho, Wo, Cout, Cin, 1, cls, n, mode, false,
+                        2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW, st);
+}
+// the input box of a forward pass is at most 256 pixels wide before its stride; the input gradient has stride^2 classes
+bool conv_strided_eligible(int Cin, int Cout, long long pixels, int kH, int kW, int stride) {
+    return conv_eligible(Cin, Cout, pixels) && stride == 2 && kH * kW <= 64 && kH <= 16 && kW <= 16;
+}
+
+int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W, int Cin, int Cout, int kH, int kW, int stride, int pad,
                  int mode, cudaStream_t st) {
-    const int Ho = H + 2 * pad - kH + 1, Wo = W + 2 * pad - kW + 1;
-    if (Ho <= 0 || Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((Cin & 31) || (Cout & 3) || Cout < 32) return NC_CUDA_ERR_UNSUPPORTED;
-    {
-        const int rc = conv_dw_halo_nhwc(dW, dy, x, N, H, W, Cin, Cout, kH, kW, pad, mode, st);
+    const int Ho = (H + 2 * pad - kH) / stride + 1, Wo = (W + 2 * pad - kW) / stride + 1;
+    if (Ho <= 0 || Wo <= 0 || stride > 2) return NC_CUDA_ERR_UNSUPPORTED;
+    if ((Cin & 3) || (Cout & 3) || Cin < 16 || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
+    const int planes = mode_planes(mode);
+    const float* xs = split_pixels(kSlotA, x, (size_t)N * H * W, Cin, mode, st);
+    const float* ds = split_pixels(kSlotB, dy, (size_t)N * Ho * Wo, Cout, mode, st);
+    if (!xs || !ds) return NC_CUDA_ERR_RUNTIME;
+    if (stride == 1) {
+        const int rc = conv_dw_halo_nhwc(dW, ds, xs, N, H, W, Cin, Cout, kH, kW, pad, planes, st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
-    const int Ncols = kH * kW * Cin;
+    const int Cp = (Cin + 31) & ~31;   // channels beyond Cin are zero-filled by TMA and dropped in the second stage
+    const int Ncols = kH * kW * Cp;
     // column tile: whole filter rows when they fit in 256 columns, else 256 / 128 / 64
     int bn_cols;
-    if (kW * Cin <= 256 && (kW * Cin) % 32 == 0 && (kW * Cin == 64 || kW * Cin == 128 || kW * Cin == 192 || kW * Cin == 256)) bn_cols = kW * Cin;
+    if (kW * Cp == 64 || kW * Cp == 128 || kW * Cp == 192 || kW * Cp == 256) bn_cols = kW * Cp;
     else bn_cols = pick_bn(Ncols);
     int bw = 1, bh = 1, bnn = 1;
-    pick_box(32, Wo, Ho, N, &bw, &bh, &bnn);
+    // split operands: a box that hung over the last image of the hi plane would read the lo plane instead of zeros
+    pick_box(32, Wo, Ho, N, &bw, &bh, &bnn, 1, 256 / stride, planes == 2);
     CUtensorMap ta, tb;
     {
-        unsigned long long dims[4] = {(unsigned long long)Cout, (unsigned long long)Wo, (unsigned long long)Ho, (unsigned long long)N};
+        unsigned long long dims[4] = {(unsigned long long)Cout, (unsigned long long)Wo, (unsigned long long)Ho, (unsigned long long)N * planes};
         unsigned long long str[3] = {(unsigned long long)Cout, (unsigned long long)Wo * Cout, (unsigned long long)Ho * Wo * Cout};
         unsigned box[4] = {32, (unsigned)bw, (unsigned)bh, (unsigned)bnn};
-        if (!make_map(&ta, dy, 4, dims, str, box, true)) return NC_CUDA_ERR_UNSUPPORTED;
-        unsigned long long xd[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N};
-        unsigned long long xs[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
-        if (!make_map(&tb, x, 4, xd, xs, box, true)) return NC_CUDA_ERR_UNSUPPORTED;
+        if (!make_map(&ta, ds, 4, dims, str, box, true)) return NC_CUDA_ERR_UNSUPPORTED;
+        unsigned long long xd[4] = {(unsigned long long)Cin, (unsigned long long)W, (unsigned long long)H, (unsigned long long)N * planes};
+        unsigned long long xst[3] = {(unsigned long long)Cin, (unsigned long long)W * Cin, (unsigned long long)H * W * Cin};
+        if (!make_map(&tb, xs, 4, xd, xst, box, true, stride)) return NC_CUDA_ERR_UNSUPPORTED;
     }
     TcParams p = {};
     p.kind = KIND_DW;
@@ -937,8 +1042,11 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
     p.bw = bw; p.bh = bh; p.bn = bnn;
     p.tiles_w = (Wo + bw - 1) / bw; p.tiles_h = (Ho + bh - 1) / bh;
     p.Ho = Ho; p.Wo = Wo; p.Nimg = N;
-    p.kW = kW; p.pad = pad; p.Cin = Cin;
-    p.num_k_tiles = p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
+    p.kW = kW; p.pad = pad; p.stride = stride; p.Cin = Cp;
+    p.passes = planes == 2 ? 3 : 1;
+    p.pass_tiles = p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
+    p.a_plane = p.b_plane = N;
+    p.num_k_tiles = p.pass_tiles * p.passes;
     p.alpha = 1.f;
     p.err = ncc::device_error_word();
     const int tiles_m = (Cout + BM - 1) / BM, tiles_n = (Ncols + bn_cols - 1) / bn_cols;
@@ -950,25 +1058,41 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
     dim3 grid(tiles_n, tiles_m, splits);
     p.flops = 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW;
     int rc;
-    if (bn_cols == 192) rc = launch_mode<192, true, true>(mode, ta, tb, p, grid, st);
-    else rc = launch_bn<true, true>(bn_cols, mode, ta, tb, p, grid, st);
+    if (bn_cols == 192) rc = launch_one<192, true, true, 1>(ta, tb, p, grid, st);
+    else rc = launch_bn<true, true>(bn_cols, ta, tb, p, grid, st);
     if (rc) return rc;
     return dw_reduce(dW, p.partial, splits, Cout, Cin, kH, kW, st);
 }
 
 int dw_reduce(float* dW, const float* partial, int splits, int Cout, int Cin, int kH, int kW, cudaStream_t st) {
-    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, dW, partial, splits, Cout, Cin, kH, kW);
+    const int Cp = (Cin + 31) & ~31;
+    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cp * kH * kW, 256), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("dw_reduce");
 }
 
-int pack_weights_fwd(float* wp, const float* w, int Cout, int Cin, int kH, int kW, bool round, cudaStream_t st) {
-    ncc::launch(pack_weights_kernel<false>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
+// Packed weights: rounded to TF32 in every tensor-core mode, with the remainders as a second plane for 3xTF32.
+int pack_weights_fwd(float* wp, const float* w, int Cout, int Cin, int kH, int kW, int planes, cudaStream_t st) {
+    if (kH * kW > 64) return NC_CUDA_ERR_UNSUPPORTED;
+    TapOrder o;
+    for (int t = 0; t < kH * kW; t++) o.at[t] = (unsigned char)t;
+    ncc::launch(pack_weights_kernel<false>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH * kW, o, 1, planes);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_fwd");
 }
-int pack_weights_dx(float* wp, const float* w, int Cout, int Cin, int kH, int kW, bool round, cudaStream_t st) {
-    ncc::launch(pack_weights_kernel<true>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH, kW, round ? 1 : 0);
+int pack_weights_dx(float* wp, const float* w, int Cout, int Cin, int kH, int kW, int stride, int pad, int planes, cudaStream_t st) {
+    if (kH * kW > 64) return NC_CUDA_ERR_UNSUPPORTED;
+    TapOrder o;
+    int t = 0;
+    for (int rh = 0; rh < stride; rh++)   // per residue class, taps reversed; stride 1: the whole filter reversed
+        for (int rw = 0; rw < stride; rw++) {
+            int a, b, th, tw, unused, outs;
+            residue_axis(rh, kH, stride, stride == 1 ? 0 : pad, 1, &a, &th, &unused, &outs);
+            residue_axis(rw, kW, stride, stride == 1 ? 0 : pad, 1, &b, &tw, &unused, &outs);
+            for (int i = th - 1; i >= 0; i--)
+                for (int j = tw - 1; j >= 0; j--) o.at[t++] = (unsigned char)((a + i * stride) * kW + b + j * stride);
+        }
+    ncc::launch(pack_weights_kernel<true>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH * kW, o, 1, planes);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_dx");
 }

@@ -68,6 +68,12 @@ __device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* tm, int 
         : "memory");
 }
 
+// untiled copy, 16-byte aligned addresses and size
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void prefetch_l2(const void* gptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(gptr)); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -155,9 +161,10 @@ inline EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// rank-2..4 f32 tensor map with 128-byte swizzle; dims/box innermost first, strides in elements for dims 1..
+// rank-2..4 f32 tensor map with 128-byte swizzle; dims/box innermost first, strides in elements for dims 1..  traverse: the box
+// takes every traverse-th element of dims 1 and 2 (a strided convolution's input pixels); box counts elements taken.
 inline bool make_map(CUtensorMap* tm, const float* base, int rank, const unsigned long long* dims,
-                     const unsigned long long* strides_elems, const unsigned* box, bool mn_major) {
+                     const unsigned long long* strides_elems, const unsigned* box, bool mn_major, int traverse = 1) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     if (reinterpret_cast<uintptr_t>(base) & 15u) return false;
@@ -165,9 +172,9 @@ inline bool make_map(CUtensorMap* tm, const float* base, int rank, const unsigne
     cuuint32_t bdim[4], estr[4];
     for (int i = 0; i < rank; i++) {
         gdim[i] = dims[i];
-        bdim[i] = box[i];
-        estr[i] = 1;
-        if (dims[i] == 0 || box[i] == 0 || box[i] > 256) return false;
+        estr[i] = (i == 1 || i == 2) && rank == 4 ? (cuuint32_t)traverse : 1u;
+        bdim[i] = box[i] * estr[i];
+        if (dims[i] == 0 || box[i] == 0 || bdim[i] > 256) return false;
     }
     for (int i = 0; i + 1 < rank; i++) {
         gstr[i] = strides_elems[i] * 4ull;

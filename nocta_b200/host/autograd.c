@@ -192,7 +192,7 @@ nc_error nc_backward(nc_tensor* t, nc_tensor* grad_output) {
     } else {
         if (t->numel != 1) { NC_SET_ERROR(NC_ERR_SHAPE_MISMATCH, "backward: output must be scalar, got %zu elements", t->numel); return NC_ERR_SHAPE_MISMATCH; }
         seed = nci_empty_on(t->shape, t->ndim, t->dtype, t->storage->device);
-        if (seed) nc_tensor_fill_(seed, 1.0);
+        if (seed && !nci_ignores_unit_seed(t->grad_fn)) nc_tensor_fill_(seed, 1.0);   /* else one launch less */
         g_unit_seed = seed;
     }
     if (!seed) return NC_ERR_ALLOC;

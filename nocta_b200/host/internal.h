@@ -52,6 +52,8 @@ bool nci_tf32_mode(void);
 bool nci_ok(int status, const char* op);
 /* g is the all-ones seed nc_backward created itself for a scalar loss (its value is known without a device read) */
 bool nci_is_unit_seed(const nc_tensor* g);
+/* the node's backward callback asks nci_is_unit_seed before it would read its gradient: the seed's memory may stay unset */
+bool nci_ignores_unit_seed(const nc_node* node);
 /* autograd wiring for an op output */
 nc_node* nci_attach(nc_tensor* out, const char* name, nc_backward_fn fn);
 void nci_strides4(const nc_tensor* t, size_t s[4]);

@@ -402,6 +402,10 @@ static nc_tensor** bwd_mse(nc_tensor* g, nc_tensor** saved, size_t n) {
     return out;
 }
 
+bool nci_ignores_unit_seed(const nc_node* node) {
+    return node && (node->backward == bwd_saved_grad || node->backward == bwd_mse || node->backward == bwd_sum_all);
+}
+
 nc_tensor* nc_cross_entropy_loss_ex(nc_tensor* logits, nc_tensor* targets, nc_reduction reduction) {
     if (!nci_need_cuda_f32(logits, "cross_entropy")) return NULL;
     if (!targets) { NC_SET_ERROR(NC_ERR_NULL_PTR, "cross_entropy: null targets"); return NULL; }
