@@ -159,14 +159,21 @@ dw_kernel(float* __restrict__ dW, float* __restrict__ db, const float* __restric
             for (int r = rg; r < g.Ho; r += rgroups) {
                 const float* xr = xt + ci * xper + (r + kh) * g.pitch;
                 const float* dr = dt + co * dper + r * dpitch;
+                int w = 0;
 #pragma unroll 2
-                for (int w = 0; w < dpitch; w += 4) {
+                for (; w + 4 <= g.Wo; w += 4) {
                     float xv[XV];
 #pragma unroll
                     for (int j = 0; j < XV; j += 4) *reinterpret_cast<float4*>(xv + j) = *reinterpret_cast<const float4*>(xr + w + j);
                     const float4 d = *reinterpret_cast<const float4*>(dr + w);
 #pragma unroll
                     for (int j = 0; j < K; j++) acc[j] = fmaf(d.w, xv[3 + j], fmaf(d.z, xv[2 + j], fmaf(d.y, xv[1 + j], fmaf(d.x, xv[j], acc[j]))));
+                }
+                // one by one: a zero of the padding times an infinity further along the row would be a NaN in taps that never see it
+                for (; w < g.Wo; w++) {
+                    const float d = dr[w];
+#pragma unroll
+                    for (int j = 0; j < K; j++) acc[j] = fmaf(d, xr[w + j], acc[j]);
                 }
             }
         }

@@ -690,8 +690,9 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, 
     }
 }
 
-// dst[plane][tap][out][in], `in` the channels of the reduction; tap t takes filter position at[t].  DX: out = ci, in = co.
-struct TapOrder { unsigned char at[64]; };
+// dst[plane][tap][out][in], `in` the channels of the reduction.  DX: out = ci, in = co.  Tap t takes filter position t, counted from
+// the end for DX; for strided layers (at most 64 taps) position at[t].
+struct TapOrder { int listed; unsigned char at[64]; };
 template <bool DX>
 __global__ void __launch_bounds__(256) pack_weights_kernel(float* __restrict__ wp, const float* __restrict__ w, int Cout, int Cin,
                                                            int T, const __grid_constant__ TapOrder order, int round, int planes) {
@@ -702,7 +703,8 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(float* __restrict__ w
         int co, ci;
         if (!DX) { ci = r % Cin; r /= Cin; co = r % Cout; r /= Cout; }
         else { co = r % Cout; r /= Cout; ci = r % Cin; r /= Cin; }
-        const float v = w[((size_t)co * Cin + ci) * T + order.at[r]];
+        const int tap = order.listed ? order.at[r] : (DX ? T - 1 - (int)r : (int)r);
+        const float v = w[((size_t)co * Cin + ci) * T + tap];
         const float h = round ? ncc::round_tf32(v) : v;
         wp[i] = h;
         if (planes == 2) wp[total + i] = ncc::round_tf32(v - h);
@@ -1073,25 +1075,26 @@ int dw_reduce(float* dW, const float* partial, int splits, int Cout, int Cin, in
 
 // Packed weights: rounded to TF32 in every tensor-core mode, with the remainders as a second plane for 3xTF32.
 int pack_weights_fwd(float* wp, const float* w, int Cout, int Cin, int kH, int kW, int planes, cudaStream_t st) {
-    if (kH * kW > 64) return NC_CUDA_ERR_UNSUPPORTED;
-    TapOrder o;
-    for (int t = 0; t < kH * kW; t++) o.at[t] = (unsigned char)t;
+    const TapOrder o = {};
     ncc::launch(pack_weights_kernel<false>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH * kW, o, 1, planes);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_fwd");
 }
 int pack_weights_dx(float* wp, const float* w, int Cout, int Cin, int kH, int kW, int stride, int pad, int planes, cudaStream_t st) {
-    if (kH * kW > 64) return NC_CUDA_ERR_UNSUPPORTED;
-    TapOrder o;
-    int t = 0;
-    for (int rh = 0; rh < stride; rh++)   // per residue class, taps reversed; stride 1: the whole filter reversed
-        for (int rw = 0; rw < stride; rw++) {
-            int a, b, th, tw, unused, outs;
-            residue_axis(rh, kH, stride, stride == 1 ? 0 : pad, 1, &a, &th, &unused, &outs);
-            residue_axis(rw, kW, stride, stride == 1 ? 0 : pad, 1, &b, &tw, &unused, &outs);
-            for (int i = th - 1; i >= 0; i--)
-                for (int j = tw - 1; j >= 0; j--) o.at[t++] = (unsigned char)((a + i * stride) * kW + b + j * stride);
-        }
+    TapOrder o = {};
+    if (stride > 1) {   // per residue class, taps reversed
+        if (kH * kW > 64) return NC_CUDA_ERR_UNSUPPORTED;
+        o.listed = 1;
+        int t = 0;
+        for (int rh = 0; rh < stride; rh++)
+            for (int rw = 0; rw < stride; rw++) {
+                int a, b, th, tw, unused, outs;
+                residue_axis(rh, kH, stride, pad, 1, &a, &th, &unused, &outs);
+                residue_axis(rw, kW, stride, pad, 1, &b, &tw, &unused, &outs);
+                for (int i = th - 1; i >= 0; i--)
+                    for (int j = tw - 1; j >= 0; j--) o.at[t++] = (unsigned char)((a + i * stride) * kW + b + j * stride);
+            }
+    }
     ncc::launch(pack_weights_kernel<true>, ncc::grid_for((long long)Cout * Cin * kH * kW, 256), 256, 0, st, wp, w, Cout, Cin, kH * kW, o, 1, planes);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("pack_weights_dx");
