@@ -38,8 +38,9 @@ __device__ __forceinline__ void stage_image(float* tile, const float* __restrict
 
 // A thread owns kPX pixels x 4 output channels over the input channels ci = slice, slice + slices, ...; the slices of one output
 // are added through shared memory in slice order, which also puts consecutive channels on consecutive threads for the store.
-constexpr int kPX = 4;
-template <int K>
+// A forward pass is not sliced but takes fewer pixels per thread: its sums then run in the order of the general path, and the
+// ReLU and max-pool decisions behind it come out the same whichever of the two takes the layer.
+template <int K, int kPX>
 __global__ void __launch_bounds__(256) conv_kernel(float* __restrict__ y, const float* __restrict__ x, const float* __restrict__ w,
                                                    const float* __restrict__ bias, Geo g, int flip, int slices) {
     ncc::pdl_wait();
@@ -235,13 +236,13 @@ Geo make(int N, int Cin, int H, int W, int Cout, int k, int pad, const long long
     return g;
 }
 
-template <int K>
+template <int K, int kPX>
 int launch_conv(float* y, const float* x, const float* w, const float* bias, Geo g, bool flip, cudaStream_t st) {
     g.pitch = (g.Wo + kPX - 1) / kPX * kPX + K - 1;   // the last pixel group may read beyond the image: zeros
     g.in_rows = g.rows + K - 1;
     const int items = g.rows * ((g.Wo + kPX - 1) / kPX) * g.cog;
-    // slices of the input channels until the 256 threads of a block have work
-    int slices = 256 / items;
+    // input gradient: slices of the channels until the 256 threads of a block have work
+    int slices = flip ? 256 / items : 1;
     if (slices > g.Cin) slices = g.Cin;
     if (slices < 1) slices = 1;
     const size_t tile = (((size_t)g.Cin * g.in_rows * g.pitch) + 3) & ~(size_t)3;
@@ -249,10 +250,18 @@ int launch_conv(float* y, const float* x, const float* w, const float* bias, Geo
     if (slices > 1) smem += sizeof(float) * (size_t)slices * items * kPX * 4;
     if (smem > kMaxSmem || (long long)g.N * g.bands > 0x7fffffffLL) return NC_CUDA_ERR_UNSUPPORTED;
     static bool set = false;
-    if (!set) { NCC_TRY(cudaFuncSetAttribute(conv_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)); set = true; }
-    ncc::launch(conv_kernel<K>, g.N * g.bands, 256, smem, st, y, x, w, bias, g, flip ? 1 : 0, slices);
+    if (!set) { NCC_TRY(cudaFuncSetAttribute(conv_kernel<K, kPX>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)); set = true; }
+    ncc::launch(conv_kernel<K, kPX>, g.N * g.bands, 256, smem, st, y, x, w, bias, g, flip ? 1 : 0, slices);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("small_conv");
+}
+// pixels per thread: four, fewer in a forward pass whose block has no work for 256 threads then
+template <int K>
+int pick_conv(float* y, const float* x, const float* w, const float* bias, const Geo& g, bool flip, cudaStream_t st) {
+    auto items = [&](int px) { return (long long)g.rows * ((g.Wo + px - 1) / px) * g.cog; };
+    if (flip || items(2) > 256) return launch_conv<K, 4>(y, x, w, bias, g, flip, st);
+    if (items(1) > 256) return launch_conv<K, 2>(y, x, w, bias, g, flip, st);
+    return launch_conv<K, 1>(y, x, w, bias, g, flip, st);
 }
 
 template <int K>
@@ -297,9 +306,9 @@ int conv(float* y, const long long ys[4], const float* x, const long long xs[4],
     g.rows = (g.Ho + bands - 1) / bands;
     g.bands = (g.Ho + g.rows - 1) / g.rows;
     switch (k) {
-        case 3: return launch_conv<3>(y, x, w, bias, g, flip, st);
-        case 5: return launch_conv<5>(y, x, w, bias, g, flip, st);
-        case 7: return launch_conv<7>(y, x, w, bias, g, flip, st);
+        case 3: return pick_conv<3>(y, x, w, bias, g, flip, st);
+        case 5: return pick_conv<5>(y, x, w, bias, g, flip, st);
+        case 7: return pick_conv<7>(y, x, w, bias, g, flip, st);
     }
     return NC_CUDA_ERR_UNSUPPORTED;
 }

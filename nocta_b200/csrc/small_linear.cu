@@ -18,26 +18,30 @@ namespace {
 constexpr int kWarps = 8;
 
 // rows_kernel: a block owns MT rows of a, 32 rows of b (one per lane) and up to 1024 k; longer sums are split over a cluster of up
-// to eight blocks.  Every row arrives as one bulk copy, all of them in flight at once; a warp then takes an eighth of k from shared
-// memory, b one row per lane, a broadcast, with MT accumulators a thread and no exchange between lanes.  Warps, then the blocks of
-// the cluster, are added in order.
+// to eight blocks.  Every row arrives as one bulk copy, all of them in flight at once; a warp then takes one of KS slices of k from
+// shared memory, b one row per lane, a broadcast, with MR accumulators a thread and no exchange between lanes.  Slices, then the
+// blocks of the cluster, are added in order.  KS = 8, all warps along k, but for sums of up to 256 the slices are those of the
+// general path (simt_matmul: none below 256, then of 64) and the other warps take other rows: the layers of small networks get the
+// same sums from both, and so the same ReLU decisions.
 // Bound by reading b and by the copy engine: whole rows (4 KB) per copy; with a copy per row and warp (512 bytes) the same kernel
 // took 11 us for 16 rows against 4096 x 1024 weights, as did loads into registers with k across the lanes; 64 x 64 tiles 53 us.
 constexpr int kSlice = 128;   // k per warp at most
 
-template <int MT>
+template <int MT, int KS>
 __global__ void __launch_bounds__(kWarps * 32) rows_kernel(float* __restrict__ d, long long ldd, const float* __restrict__ a, long long lda,
                                                            const float* __restrict__ b, long long ldb, const float* __restrict__ bias,
                                                            int M, int N, int K, int slice, int wpitch, int blocks_k, int round_b,
                                                            unsigned int* err) {
-    extern __shared__ __align__(128) float sm[];   // a [MT][8 * slice], b [32][wpitch]
-    __shared__ float red[kWarps][MT][32];
+    extern __shared__ __align__(128) float sm[];   // a [MT][KS * slice], b [32][wpitch]
+    constexpr int MR = MT * KS / kWarps;           // rows a warp sums
+    static_assert(MR >= 1, "a row per warp");
+    __shared__ float red[KS][MT][32];
     __shared__ __align__(8) uint64_t bar;
     __shared__ int abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = kWarps * slice;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = KS * slice, ks = warp % KS, r0 = warp / KS * MR;
     const int n = blockIdx.x / blocks_k * 32 + lane, m0 = blockIdx.y * MT;
     const int k0 = (int)(blockIdx.x % blocks_k) * chunk, kb = (K - k0) < chunk ? (K - k0) : chunk;   // this block's k
-    const int kn = (kb - warp * slice) < slice ? (kb - warp * slice) : slice;                        // this warp's; may be <= 0
+    const int kn = (kb - ks * slice) < slice ? (kb - ks * slice) : slice;                            // this warp's; may be <= 0
     float* xs = sm;
     float* ws = sm + MT * chunk;
     if (threadIdx.x == 0) {
@@ -56,18 +60,18 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(float* __restrict__ d
         if (lane < rows_b) tc::bulk_copy(tc::smem_u32(ws + lane * wpitch), b + (long long)n * ldb + k0, bytes, full);
         if (lane < rows_a) tc::bulk_copy(tc::smem_u32(xs + lane * chunk), a + (long long)(m0 + lane) * lda + k0, bytes, full);
     }
-    float acc[MT];
+    float acc[MR];
 #pragma unroll
-    for (int m = 0; m < MT; m++) acc[m] = 0.f;
+    for (int m = 0; m < MR; m++) acc[m] = 0.f;
     if (tc::mbar_wait(full, 0u, err, 0xD00u, &abort_flag)) {
-        const float4* wq = reinterpret_cast<const float4*>(ws + lane * wpitch + warp * slice);
-        const float4* xq = reinterpret_cast<const float4*>(xs + warp * slice);
+        const float4* wq = reinterpret_cast<const float4*>(ws + lane * wpitch + ks * slice);
+        const float4* xq = reinterpret_cast<const float4*>(xs + r0 * chunk + ks * slice);
 #pragma unroll 4
         for (int q = 0; q < kn >> 2; q++) {
             float4 w = wq[q];
             if (round_b) w = make_float4(round_tf32(w.x), round_tf32(w.y), round_tf32(w.z), round_tf32(w.w));
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
+            for (int m = 0; m < MR; m++) {
                 const float4 x = xq[m * (chunk >> 2) + q];
                 acc[m] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc[m]))));
             }
@@ -77,12 +81,12 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(float* __restrict__ d
         while (tc::global_ns() - t0 < 2000000ull) { }
     }
 #pragma unroll
-    for (int m = 0; m < MT; m++) red[warp][m][lane] = acc[m];
+    for (int m = 0; m < MR; m++) red[ks][r0 + m][lane] = acc[m];
     __syncthreads();
     for (int i = threadIdx.x; i < MT * 32; i += kWarps * 32) {
         float s = 0.f;
 #pragma unroll
-        for (int w = 0; w < kWarps; w++) s += red[w][i >> 5][i & 31];
+        for (int w = 0; w < KS; w++) s += red[w][i >> 5][i & 31];
         red[0][i >> 5][i & 31] = s;   // only this thread reads it before
         const int m = m0 + (i >> 5), nn = n - lane + (i & 31);
         if (blocks_k == 1 && m < M && nn < N) d[(long long)m * ldd + nn] = s + (bias ? bias[nn] : 0.f);
@@ -245,16 +249,16 @@ inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) 
 
 }  // namespace
 
-template <int MT>
+template <int MT, int KS>
 static int launch_rows(float* d, long long ldd, const float* a, long long lda, const float* b, long long ldb, const float* bias, int M,
                        int N, int K, bool round_b, cudaStream_t st) {
     const int blocks_k = (K + kWarps * kSlice - 1) / (kWarps * kSlice);   // 1 .. 8
-    const int slice = ((K + blocks_k * kWarps - 1) / (blocks_k * kWarps) + 3) & ~3;
-    const int chunk = kWarps * slice, wpitch = chunk + 4;   // an odd number of 16-byte pieces: lanes read without bank conflicts
+    const int slice = ((K + blocks_k * KS - 1) / (blocks_k * KS) + 3) & ~3;
+    const int chunk = KS * slice, wpitch = chunk + (chunk % 8 == 0 ? 4 : 0);   // an odd number of 16-byte pieces: lanes read without bank conflicts
     const size_t smem = sizeof(float) * (size_t)(MT * chunk + 32 * wpitch);
     static bool set = false;
-    if (!set) { NCC_TRY(cudaFuncSetAttribute(rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024)); set = true; }
-    launch_clusters((unsigned)blocks_k, rows_kernel<MT>, dim3((unsigned)((N + 31) / 32 * blocks_k), (unsigned)((M + MT - 1) / MT)), kWarps * 32,
+    if (!set) { NCC_TRY(cudaFuncSetAttribute(rows_kernel<MT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024)); set = true; }
+    launch_clusters((unsigned)blocks_k, rows_kernel<MT, KS>, dim3((unsigned)((N + 31) / 32 * blocks_k), (unsigned)((M + MT - 1) / MT)), kWarps * 32,
                     smem, st, d, ldd, a, lda, b, ldb, bias, M, N, K, slice, wpitch, blocks_k, round_b ? 1 : 0, device_error_word());
     NCC_COUNT_LAUNCH();
     return launch_status("small_rows");
@@ -264,10 +268,14 @@ int small_rows(float* d, long long ldd, const float* a, long long lda, const flo
                int K, bool round_b, cudaStream_t st) {
     // bulk copies want 16-byte pieces; beyond eight blocks of a cluster the sum would need another level
     if (K % 4 == 0 && lda % 4 == 0 && ldb % 4 == 0 && al16(a) && al16(b) && K <= 8 * kWarps * kSlice && (M + 15) / 16 <= 65535) {
-        if (M <= 1) return launch_rows<1>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
-        if (M <= 4) return launch_rows<4>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
-        if (M <= 8) return launch_rows<8>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
-        return launch_rows<16>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        if (M <= 1) return launch_rows<1, 8>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        if (K < 256) return M <= 8 ? launch_rows<8, 1>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st)
+                                   : launch_rows<16, 1>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        if (K == 256) return M <= 8 ? launch_rows<8, 4>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st)
+                                    : launch_rows<16, 4>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        if (M <= 4) return launch_rows<4, 8>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        if (M <= 8) return launch_rows<8, 8>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
+        return launch_rows<16, 8>(d, ldd, a, lda, b, ldb, bias, M, N, K, round_b, st);
     }
     const long long row_tiles = (M + 7) / 8, groups = (N + 3) / 4;
     if (row_tiles > 65535) return set_status(NC_CUDA_ERR_UNSUPPORTED, "small_rows: %d rows", M);
