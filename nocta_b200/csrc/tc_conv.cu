@@ -918,12 +918,15 @@ int conv_halo_nhwc(float* y, const float* x, const float* wpacked, const float* 
     // M only); other images lower than 24 rows run faster on the per-tap kernel, whose 256-pixel boxes span several images.
     const bool dual = Ho == 16 && (N % 2 == 0) && Cout > 96;
     if (Ho < 24 && !dual) return NC_CUDA_ERR_UNSUPPORTED;
+    // 3xTF32 only with the pixels on M, where the reduction is spread over two accumulators, and whole chunks: the other forms
+    // accumulate longer than the per-tap kernel, which adds short segments in registers
     // Pixels on M for up to 96 output channels (measured on the 64-channel 64 x 64 layer at batch 256: 447 against 344
     // TFLOP/s with the channels on M); from 128 channels on, channels on M with N = 256 pixels is the faster shape
     // (698 against 636 TFLOP/s on the 128-channel 32 x 32 layer).
     const int ncol = (Cout + 31) & ~31;
     const bool pxm = Cout <= 96 && (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15u) == 0) &&
                      (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
+    if (planes == 2 && (!pxm || (Cin % 32) || (Cout % 32))) return NC_CUDA_ERR_UNSUPPORTED;
     CUtensorMap tw, tx;
     unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)kH * kW * Cout * planes};
     unsigned long long ws[1] = {(unsigned long long)Cin};
@@ -1008,7 +1011,8 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
     const int Ho = H + 2 * pad - kH + 1, Wo = W + 2 * pad - kW + 1;
     if (kH < 1 || kW < 2 || kH > 3 || kW > 3 || Ho <= 0 || Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
     if ((Cin % 4) || (Cout % 4) || Cin < 16 || Cout < 16) return NC_CUDA_ERR_UNSUPPORTED;
-    if ((long long)N * Ho * Wo < 4096) return NC_CUDA_ERR_UNSUPPORTED;   // too few pixels to split over the GPU
+    if ((long long)N * Ho * Wo < (planes == 2 ? 16384 : 4096)) return NC_CUDA_ERR_UNSUPPORTED;   // too few pixels to split over the GPU
+    if (planes == 2 && ((Cin % 32) || (Cout % 32))) return NC_CUDA_ERR_UNSUPPORTED;
     const bool shift = (Cin % 128) != 0;
     DwhParams p = {};
     const int Cp = (Cin + 31) & ~31;
@@ -1051,6 +1055,9 @@ int conv_dw_halo_nhwc(float* dW, const float* dy, const float* x, int N, int H, 
     const int sms = ncc::sm_count();
     int splits = sms / p.items;
     if (splits < 1) splits = 1;
+    // 3xTF32: a quarter of the pixels per accumulator, as the tensor core's accumulation is the largest error left in that mode
+    // (products of one sign, 16384 pixels: 6.9e-6 with one wave of splits, 1.5e-6 with four)
+    if (planes == 2) splits *= 4;
     if (splits > p.units_total / 4) splits = p.units_total / 4 > 0 ? p.units_total / 4 : 1;
     p.units_per_split = (p.units_total + splits - 1) / splits;
     p.splits = (p.units_total + p.units_per_split - 1) / p.units_per_split;

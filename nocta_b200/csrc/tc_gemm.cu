@@ -19,9 +19,12 @@
 //          boxes; both operands MN-major; split over the reduction with an ordered second stage.
 //
 // The kernel multiplies TF32 operands as they lie in memory.  The accuracy modes are prepared in memory: operands rounded to
-// nearest TF32, or for 3xTF32 split into two planes hi and lo (split_operand), and the reduction then runs over three passes,
-// lo * hi, hi * lo, hi * hi: to the kernel a reduction three times as long with other tile coordinates.  The small products come
-// first, so the accumulator is rounded at full size only by the last third of the additions.
+// nearest TF32, or for 3xTF32 split into two planes hi and lo (split_operand); a stage then holds both planes of both operands
+// (read once for three products: with one product per stage the loads from L2, not the tensor cores, set the pace; VGG step at batch
+// 64 2724 -> 2393 us together with the faster reduction below) and every k-step is lo * hi, hi * lo, hi * hi.  The tensor core's own
+// accumulation, which truncates, is the largest error left in that mode (5e-8 of the result per addition of eight products when all
+// have one sign: 1e-5 over K = 4096), so a segment is two reduction tiles long, and the epilogue warps add the segments in
+// registers, rounding to nearest, while the next one is multiplied: 5e-7 for any K.
 //
 // CTA = 6 warps (kernels with an MN-major operand add up to five more TMA-issuing warps): warp 0 issues TMA, warp 1
 // allocates TMEM and issues MMAs (one lane), warps 2-5 run the epilogue (tcgen05.ld -> registers -> global).
@@ -51,7 +54,8 @@ constexpr int kMaxClasses = 4;
 struct TcParams {
     int kind;
     int M, N;              // logical output extent (store masks)
-    int passes, pass_tiles;// reduction passes (1, or 3 over split operands) of pass_tiles tiles each
+    int planes;            // 1, or 2 for split operands
+    int segment;           // reduction tiles per segment (all of them unless SPLIT)
     int a_plane, b_plane;  // coordinate distance of the lo plane of A and B (rows, or images)
     int num_k_tiles;       // reduction tiles in total
     int k_tiles_per_split; // reduction tiles per blockIdx.z
@@ -90,18 +94,20 @@ constexpr int CHUNK_BYTES = 32 * BK * 4;  // one 32 x 32 MN-major chunk: 4 KB
 constexpr int kMaxStages = 8;
 constexpr int kSmemBudget = 196 * 1024;  // one persistent CTA per SM
 
-// NACC accumulators take the k-steps in turn and are added in f32 by the epilogue: the 3xTF32 GEMM spreads its additions over two,
-// because the tensor core's own accumulation is the largest error term left in that mode.
-template <int BN, int NACC>
+constexpr int kSegment = 2;             // reduction tiles per segment of a 3xTF32 product
+
+template <int BN, bool SPLIT>
 struct TileCfg {
+    static constexpr int PLANES = SPLIT ? 2 : 1;
     static constexpr int B_BYTES = BN * BK * 4;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int B_AT = PLANES * A_BYTES;   // stage: the planes (hi, lo) of A, then those of B
+    static constexpr int STAGE_BYTES = PLANES * (A_BYTES + B_BYTES);
     static constexpr int STAGES_RAW = kSmemBudget / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > kMaxStages ? kMaxStages : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;  // + alignment slack
     static constexpr int ACC_COLS = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
-    static constexpr int NBUF = 2;   // the epilogue of one tile overlaps the MMAs of the next
-    static constexpr int TMEM_COLS = ACC_COLS * NACC * NBUF;
+    static constexpr int NBUF = 2;   // the epilogue of one tile (or segment) overlaps the MMAs of the next
+    static constexpr int TMEM_COLS = ACC_COLS * NBUF;
     static_assert(TMEM_COLS <= 512, "tensor memory");
 };
 
@@ -136,15 +142,21 @@ __device__ __forceinline__ Tile tile_of(const TcParams& p, int t) {
     if (p.kind == KIND_CONVT) {
         while (o.cls + 1 < p.classes && o.n_tile >= p.cls[o.cls + 1].tile0) o.cls++;
         o.px = o.n_tile - p.cls[o.cls].tile0;
-        o.kt_end = p.cls[o.cls].kH * p.cls[o.cls].kW * p.cchunks * p.passes;   // never split
+        o.kt_end = p.cls[o.cls].kH * p.cls[o.cls].kW * p.cchunks;   // never split
     }
     return o;
 }
 
-template <int BN, bool A_MN, bool B_MN, int NACC>
-__global__ void __launch_bounds__(352, 1)
+// reduction tiles of the segment that starts at kt
+__device__ __forceinline__ int segment_tiles(const TcParams& p, const Tile& T, int kt) {
+    return (T.kt_end - kt) < p.segment ? (T.kt_end - kt) : p.segment;
+}
+
+// SPLIT: operands in two planes, segments added in registers (3xTF32)
+template <int BN, bool A_MN, bool B_MN, bool SPLIT>
+__global__ void __launch_bounds__(ProdCfg<A_MN, B_MN, BN>::THREADS, 1)
 tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TcParams p) {
-    using Cfg = TileCfg<BN, NACC>;
+    using Cfg = TileCfg<BN, SPLIT>;
     constexpr int NBUF = Cfg::NBUF;
     const int STAGES = p.stages;
     extern __shared__ uint8_t dyn_smem[];
@@ -212,14 +224,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 int my_n = 0;                                 // copies this producer issues per stage of this tile
                 for (int c = own; c < (forA ? NACH : NBCH); c += step) my_n += (32 * c < edge) ? 1 : 0;
                 const bool chunked = forA ? A_MN : B_MN;
-                const uint32_t my_bytes = chunked ? (uint32_t)my_n * CHUNK_BYTES : (forA ? (uint32_t)A_BYTES : (uint32_t)Cfg::B_BYTES);
-                int pass = T.kt_begin / p.pass_tiles, lk = T.kt_begin - pass * p.pass_tiles;
+                const uint32_t my_bytes = Cfg::PLANES * (chunked ? (uint32_t)my_n * CHUNK_BYTES : (forA ? (uint32_t)A_BYTES : (uint32_t)Cfg::B_BYTES));
                 int dtw = 0, dth = 0, dtn = 0;
                 // DW: (first channel, tap) of this producer's B chunks
                 int ci0[4] = {0, 0, 0, 0}, dkh[4] = {0, 0, 0, 0}, dkw[4] = {0, 0, 0, 0};
                 if (p.kind == KIND_DW) {
-                    dtw = lk % p.tiles_w;
-                    const int tt = lk / p.tiles_w;
+                    dtw = T.kt_begin % p.tiles_w;
+                    const int tt = T.kt_begin / p.tiles_w;
                     dth = tt % p.tiles_h; dtn = tt / p.tiles_h;
                     if (!forA) {
 #pragma unroll
@@ -234,48 +245,50 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 for (int kt = T.kt_begin; kt < T.kt_end; kt++) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, p.err, 0x100u + s, abortp)) { ok = false; break; }
                     const uint32_t full = smem_u32(&bar_full[s]);
-                    const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES;
-                    const uint32_t b_dst = a_dst + A_BYTES;
-                    // split operands: passes lo * hi, hi * lo, hi * hi
-                    const int off = p.passes == 1 ? 0 : (forA ? (pass == 0 ? p.a_plane : 0) : (pass == 1 ? p.b_plane : 0));
                     if (my_bytes == 0) {
                         mbar_arrive(full);
                     } else {
                         mbar_expect_tx(full, my_bytes);
-                        if (p.kind == KIND_GEMM) {
-                            const int k0 = lk * BK;
-                            if (forA) {
-                                if (!A_MN) tma_2d(a_dst, &tmA, k0, m0 + off, full);
-                                else {
+#pragma unroll
+                        for (int pl = 0; pl < Cfg::PLANES; pl++) {
+                            const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES + (uint32_t)(pl * A_BYTES);
+                            const uint32_t b_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES + (uint32_t)(Cfg::B_AT + pl * Cfg::B_BYTES);
+                            const int off = pl * (forA ? p.a_plane : p.b_plane);
+                            if (p.kind == KIND_GEMM) {
+                                const int k0 = kt * BK;
+                                if (forA) {
+                                    if (!A_MN) tma_2d(a_dst, &tmA, k0, m0 + off, full);
+                                    else {
+#pragma unroll
+                                        for (int i = 0; i < 4; i++) {
+                                            const int c = own + i * step;
+                                            if (c < NACH && 32 * c < edge) tma_2d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, k0 + off, full);
+                                        }
+                                    }
+                                } else if (!B_MN) {
+                                    tma_2d(b_dst, &tmB, k0, n0 + off, full);
+                                } else {
 #pragma unroll
                                     for (int i = 0; i < 4; i++) {
                                         const int c = own + i * step;
-                                        if (c < NACH && 32 * c < edge) tma_2d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, k0 + off, full);
+                                        if (c < NBCH && 32 * c < edge) tma_2d(b_dst + c * CHUNK_BYTES, &tmB, n0 + 32 * c, k0 + off, full);
                                     }
                                 }
-                            } else if (!B_MN) {
-                                tma_2d(b_dst, &tmB, k0, n0 + off, full);
-                            } else {
+                            } else {  // KIND_DW (both operands MN-major)
+                                const int w0 = dtw * p.bw, h0 = dth * p.bh, nn0 = dtn * p.bn + off;
+                                if (forA) {
 #pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const int c = own + i * step;
-                                    if (c < NBCH && 32 * c < edge) tma_2d(b_dst + c * CHUNK_BYTES, &tmB, n0 + 32 * c, k0 + off, full);
-                                }
-                            }
-                        } else {  // KIND_DW (both operands MN-major)
-                            const int w0 = dtw * p.bw, h0 = dth * p.bh, nn0 = dtn * p.bn + off;
-                            if (forA) {
+                                    for (int i = 0; i < 4; i++) {
+                                        const int c = own + i * step;
+                                        if (c < NACH && 32 * c < edge) tma_4d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, w0, h0, nn0, full);
+                                    }
+                                } else {
 #pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const int c = own + i * step;
-                                    if (c < NACH && 32 * c < edge) tma_4d(a_dst + c * CHUNK_BYTES, &tmA, m0 + 32 * c, w0, h0, nn0, full);
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 4; i++) {
-                                    const int c = own + i * step;
-                                    if (c < NBCH && 32 * c < edge)
-                                        tma_4d(b_dst + c * CHUNK_BYTES, &tmB, ci0[i], w0 * p.stride + dkw[i] - p.pad, h0 * p.stride + dkh[i] - p.pad, nn0, full);
+                                    for (int i = 0; i < 4; i++) {
+                                        const int c = own + i * step;
+                                        if (c < NBCH && 32 * c < edge)
+                                            tma_4d(b_dst + c * CHUNK_BYTES, &tmB, ci0[i], w0 * p.stride + dkw[i] - p.pad, h0 * p.stride + dkh[i] - p.pad, nn0, full);
+                                    }
                                 }
                             }
                         }
@@ -283,7 +296,6 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                     if (p.kind == KIND_DW) {
                         if (++dtw == p.tiles_w) { dtw = 0; if (++dth == p.tiles_h) { dth = 0; dtn++; } }
                     }
-                    if (++lk == p.pass_tiles) { lk = 0; pass++; dtw = 0; dth = 0; dtn = 0; }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
             }
@@ -299,48 +311,40 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 const Tile T = tile_of(p, t);
                 const int m0 = T.m0, n0 = T.n_tile * BN;
-                int pass = 0, lk = 0;
                 // pixel box of this tile (CONV: the m tile, CONVT: the n tile), running (tap, chunk)
-                int pw0 = 0, ph0 = 0, pn0 = 0, cc = 0, kh = 0, kw = 0, shift = 0, kWc = p.kW, taps_left = 0, wrow0 = 0, taps = 0;
+                int pw0 = 0, ph0 = 0, pn0 = 0, cc = 0, kh = 0, kw = 0, shift = 0, kWc = p.kW, wrow0 = 0;
                 if (p.kind == KIND_CONV) {
                     const int pt = m0 / BM, tw = pt % p.tiles_w, tt = pt / p.tiles_w;
                     pw0 = tw * p.bw - p.pad; ph0 = (tt % p.tiles_h) * p.bh - p.pad; pn0 = (tt / p.tiles_h) * p.bn;
-                    taps = p.pass_tiles / p.cchunks;
                 } else if (p.kind == KIND_CONVT) {
                     const ConvClass& c = p.cls[T.cls];
                     const int tw = T.px % c.tiles_w, tt = T.px / c.tiles_w;
                     pw0 = tw * p.bw * p.stride - c.pad_w; ph0 = (tt % c.tiles_h) * p.bh * p.stride - c.pad_h; pn0 = (tt / c.tiles_h) * p.bn;
                     kWc = c.kW; wrow0 = c.wrow0;
-                    taps = c.kH * c.kW;
-                } else {
-                    pass = T.kt_begin / p.pass_tiles; lk = T.kt_begin - pass * p.pass_tiles;
                 }
-                taps_left = taps;
                 for (int kt = T.kt_begin; kt < T.kt_end; kt++) {
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, p.err, 0x100u + s, abortp)) { ok = false; break; }
                     const uint32_t full = smem_u32(&bar_full[s]);
                     mbar_expect_tx(full, (uint32_t)Cfg::STAGE_BYTES);
-                    const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES;
-                    const uint32_t b_dst = a_dst + A_BYTES;
-                    const int offA = (p.passes == 3 && pass == 0) ? p.a_plane : 0, offB = (p.passes == 3 && pass == 1) ? p.b_plane : 0;
-                    if (p.kind == KIND_GEMM) {
-                        const int k0 = lk * BK;
-                        tma_2d(a_dst, &tmA, k0, m0 + offA, full);
-                        tma_2d(b_dst, &tmB, k0, n0 + offB, full);
-                        if (++lk == p.pass_tiles) { lk = 0; pass++; }
-                    } else {
-                        if (p.kind == KIND_CONV) {
+#pragma unroll
+                    for (int pl = 0; pl < Cfg::PLANES; pl++) {
+                        const uint32_t a_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES + (uint32_t)(pl * A_BYTES);
+                        const uint32_t b_dst = tiles_base + (uint32_t)s * Cfg::STAGE_BYTES + (uint32_t)(Cfg::B_AT + pl * Cfg::B_BYTES);
+                        const int offA = pl * p.a_plane, offB = pl * p.b_plane;
+                        if (p.kind == KIND_GEMM) {
+                            tma_2d(a_dst, &tmA, kt * BK, m0 + offA, full);
+                            tma_2d(b_dst, &tmB, kt * BK, n0 + offB, full);
+                        } else if (p.kind == KIND_CONV) {
                             tma_4d(a_dst, &tmA, cc * 32, pw0 + kw, ph0 + kh, pn0 + offA, full);
                             tma_2d(b_dst, &tmB, cc * 32, shift * p.wrows + n0 + offB, full);
                         } else {
                             tma_2d(a_dst, &tmA, cc * 32, wrow0 + shift * p.wrows + m0 + offA, full);
                             tma_4d(b_dst, &tmB, cc * 32, pw0 + kw, ph0 + kh, pn0 + offB, full);
                         }
-                        if (++cc == p.cchunks) {
-                            cc = 0; shift++;
-                            if (++kw == kWc) { kw = 0; kh++; }
-                            if (--taps_left == 0) { taps_left = taps; shift = 0; kh = 0; kw = 0; pass++; }
-                        }
+                    }
+                    if (p.kind != KIND_GEMM && ++cc == p.cchunks) {
+                        cc = 0; shift++;
+                        if (++kw == kWc) { kw = 0; kh++; }
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1u; }
                 }
@@ -362,7 +366,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             const uint32_t kstep_a = A_MN ? 1024u : 32u, kstep_b = B_MN ? 1024u : 32u;
             // descriptors are built once; a ring slot or k-step only moves the 14-bit start-address field
             const uint64_t da0 = smem_desc(tiles_base, lbo_a, sbo_a, lay_a);
-            const uint64_t db0 = smem_desc(tiles_base + A_BYTES, lbo_b, sbo_b, lay_b);
+            const uint64_t db0 = smem_desc(tiles_base + Cfg::B_AT, lbo_b, sbo_b, lay_b);
             int s = 0;
             uint32_t ph = 0, tile_iter = 0;
             bool ok = true;
@@ -371,33 +375,43 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             // are issued and only looked at afterwards: with the producers ahead it is already set, and the wait at
             // the top of the next round is skipped.
             bool known_ready = false;
-            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, tile_iter++) {
+            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 const Tile T = tile_of(p, t);
-                const int nk = T.kt_end - T.kt_begin;
-                const uint32_t ab = tile_iter % NBUF;
-                // wait until the epilogue has drained this accumulator buffer (first use passes at once)
-                if (!mbar_wait(smem_u32(&bar_acc_empty[ab]), ((tile_iter / NBUF) & 1u) ^ 1u, p.err, 0x500u + ab, abortp)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t acc_base = tmem_base + ab * (uint32_t)(NACC * Cfg::ACC_COLS);
-                for (int i = 0; i < nk; i++) {
-                    if (!known_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, p.err, 0x200u + s, abortp)) { ok = false; break; }
+                int kt = T.kt_begin;
+                do {   // once also for a tile without reduction
+                    const int nk = segment_tiles(p, T, kt);
+                    const uint32_t ab = tile_iter % NBUF;
+                    // wait until the epilogue has drained this accumulator buffer (first use passes at once)
+                    if (!mbar_wait(smem_u32(&bar_acc_empty[ab]), ((tile_iter / NBUF) & 1u) ^ 1u, p.err, 0x500u + ab, abortp)) { ok = false; break; }
                     tc_fence_after();
-                    {
-                        const int s1 = (s + 1 == STAGES) ? 0 : s + 1;
-                        const uint32_t ph1 = (s + 1 == STAGES) ? (ph ^ 1u) : ph;
-                        known_ready = mbar_test(smem_u32(&bar_full[s1]), ph1);
-                    }
-                    const uint64_t soff = (uint64_t)(((uint32_t)s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
+                    const uint32_t acc = tmem_base + ab * (uint32_t)Cfg::ACC_COLS;
+                    for (int i = 0; i < nk; i++) {
+                        if (!known_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, p.err, 0x200u + s, abortp)) { ok = false; break; }
+                        tc_fence_after();
+                        {
+                            const int s1 = (s + 1 == STAGES) ? 0 : s + 1;
+                            const uint32_t ph1 = (s + 1 == STAGES) ? (ph ^ 1u) : ph;
+                            known_ready = mbar_test(smem_u32(&bar_full[s1]), ph1);
+                        }
+                        const uint64_t soff = (uint64_t)(((uint32_t)s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
 #pragma unroll
-                    for (int ks = 0; ks < BK / 8; ks++) {
-                        const uint64_t da = da0 + soff + (uint64_t)((ks * kstep_a) >> 4);
-                        const uint64_t db = db0 + soff + (uint64_t)((ks * kstep_b) >> 4);
-                        umma_tf32(acc_base + (uint32_t)((ks % NACC) * Cfg::ACC_COLS), da, db, idesc, (uint32_t)(i != 0 || ks >= NACC));
+                        for (int ks = 0; ks < BK / 8; ks++) {
+                            const uint64_t da = da0 + soff + (uint64_t)((ks * kstep_a) >> 4);
+                            const uint64_t db = db0 + soff + (uint64_t)((ks * kstep_b) >> 4);
+                            if (SPLIT) {
+                                umma_tf32(acc, da + (uint64_t)(A_BYTES >> 4), db, idesc, (uint32_t)(i != 0 || ks != 0));
+                                umma_tf32(acc, da, db + (uint64_t)(Cfg::B_BYTES >> 4), idesc, 1u);
+                            }
+                            umma_tf32(acc, da, db, idesc, (uint32_t)(SPLIT || i != 0 || ks != 0));
+                        }
+                        umma_commit(smem_u32(&bar_empty[s]));
+                        if (++s == STAGES) { s = 0; ph ^= 1u; }
                     }
-                    umma_commit(smem_u32(&bar_empty[s]));
-                    if (++s == STAGES) { s = 0; ph ^= 1u; }
-                }
-                if (ok) umma_commit(smem_u32(&bar_acc_full[ab]));
+                    if (!ok) break;
+                    umma_commit(smem_u32(&bar_acc_full[ab]));
+                    tile_iter++;
+                    kt += p.segment;
+                } while (kt < T.kt_end);
             }
         }
     } else if (warp < 6) {
@@ -415,7 +429,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                     double* sd = p.stat + ((size_t)blockIdx.x * p.M + mt * BM + r) * 2;
                     sd[0] = 0.0; sd[1] = 0.0;
                 }
-        for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, tile_iter++) {
+        for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
             const Tile T = tile_of(p, t);
             const int m0 = T.m0, n0 = T.n_tile * BN;
             if (p.kind == KIND_CONVT && p.stat && m0 != stat_m0) {
@@ -425,27 +439,51 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 }
                 ssum = 0.0; ssq = 0.0; stat_m0 = m0;
             }
-            const uint32_t ab = tile_iter % NBUF;
-            ok = mbar_wait(smem_u32(&bar_acc_full[ab]), (tile_iter / NBUF) & 1u, p.err, 0x400u + ab, abortp);
-            // all 32 lanes of a warp must agree before the aligned tcgen05.ld
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t acc_base = tmem_base + ab * (uint32_t)(NACC * Cfg::ACC_COLS) + ((uint32_t)(q * 32) << 16);
-            // 32 accumulator columns of this warp's rows; after the last chunk the buffer may be overwritten by the tile after next
-            auto read_chunk = [&](int c0, bool last, uint32_t (&v)[32]) {
-                tmem_ld32(acc_base + (uint32_t)c0, v);
-                tmem_ld_wait();
-                if (NACC > 1) {
-#pragma unroll 1
-                    for (int a = 1; a < NACC; a++) {
+            constexpr int kChunks = SPLIT ? BN / 32 : 1;
+            float sum[kChunks][32];
+#pragma unroll
+            for (int c = 0; c < kChunks; c++)
+#pragma unroll
+                for (int j = 0; j < 32; j++) sum[c][j] = 0.f;
+            uint32_t acc_base = 0, ab = 0;
+            int kt = T.kt_begin;
+            do {
+                ab = tile_iter % NBUF;
+                ok = mbar_wait(smem_u32(&bar_acc_full[ab]), (tile_iter / NBUF) & 1u, p.err, 0x400u + ab, abortp);
+                // all 32 lanes of a warp must agree before the aligned tcgen05.ld
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                acc_base = tmem_base + ab * (uint32_t)Cfg::ACC_COLS + ((uint32_t)(q * 32) << 16);
+                tile_iter++;
+                if (SPLIT) {
+#pragma unroll
+                    for (int c = 0; c < kChunks; c++) {
                         uint32_t u[32];
-                        tmem_ld32(acc_base + (uint32_t)(a * Cfg::ACC_COLS + c0), u);
+                        tmem_ld32(acc_base + (uint32_t)(c * 32), u);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+                        for (int j = 0; j < 32; j++) sum[c][j] += __uint_as_float(u[j]);
                     }
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&bar_acc_empty[ab]));
                 }
+                kt += p.segment;
+            } while (kt < T.kt_end);
+            if (!ok) break;
+            // 32 accumulator columns of this warp's rows; after the last chunk the buffer may be overwritten by the tile after next
+            auto read_chunk = [&](int c0, bool last, uint32_t (&v)[32]) {
+                if (SPLIT) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {   // chunks are asked for in order and move up: registers want constant indexes
+                        v[j] = __float_as_uint(sum[0][j]);
+#pragma unroll
+                        for (int c = 0; c + 1 < kChunks; c++) sum[c][j] = sum[c + 1][j];
+                    }
+                    return;
+                }
+                tmem_ld32(acc_base + (uint32_t)c0, v);
+                tmem_ld_wait();
                 if (last) {
                     tc_fence_before();
                     mbar_arrive(smem_u32(&bar_acc_empty[ab]));
@@ -511,8 +549,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             const bool vec_ok = ((reinterpret_cast<uintptr_t>(base) & 15u) == 0) &&
                                 (((p.partial ? (long long)p.N : p.ldd) & 3) == 0);
             // A thread holds 32 columns of ONE row, and storing them as they are would make every store instruction touch 32
-            // different lines: the block is turned through shared memory so that eight lanes store one row's 128 bytes
-            // (4096 x 4096 outputs, K = 1024: 87 -> MEASURED us).
+            // different lines: the block is turned through shared memory so that eight lanes store one row's 128 bytes.
             float (*blk)[36] = turn[q];
             const float alpha = p.partial ? 1.f : p.alpha, beta = p.partial ? 0.f : p.beta;
             const float* biasv = p.partial ? nullptr : p.bias;
@@ -638,24 +675,32 @@ static const float* split_pixels(int slot, const float* x, size_t pixels, int C,
     return mode == NC_CUDA_MATH_TF32 ? x : split_operand(slot, x, pixels, C, (size_t)C, pixels, C, mode_planes(mode), st);
 }
 
+// Sum of element i over the planes of `partial`, `plane` floats apart: in double, in order.  Eight loads are requested before the
+// first one is added.
+__device__ __forceinline__ double sum_planes(const float* __restrict__ p, int splits, size_t plane) {
+    double acc = 0.0;
+    int z = 0;
+    for (; z + 8 <= splits; z += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = p[(size_t)(z + k) * plane];
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc += (double)v[k];
+    }
+    for (; z < splits; z++) acc += (double)p[(size_t)z * plane];
+    return acc;
+}
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ D, long long ldd, const float* __restrict__ partial,
                                                             int splits, int M, int N, const float* __restrict__ bias,
                                                             float alpha, float beta) {
     ncc::pdl_wait();
     const size_t total = (size_t)M * N, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        double acc = 0.0;   // the splits are combined in double, in order: no rounding that grows with their number
-        int z = 0;
-        for (; z + 8 <= splits; z += 8) {   // eight loads requested before the first one is added
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = partial[(size_t)(z + k) * total + i];
-#pragma unroll
-            for (int k = 0; k < 8; k++) acc += (double)v[k];
-        }
-        for (; z < splits; z++) acc += (double)partial[(size_t)z * total + i];
-        const int m = (int)(i / N), n = (int)(i % N);
-        float* d = D + (size_t)m * ldd + n;
+        const double acc = sum_planes(partial + i, splits, total);
+        size_t m; int n;
+        if (total <= 0xffffffffu) { const uint32_t q = (uint32_t)i / (uint32_t)N; m = q; n = (int)((uint32_t)i - q * (uint32_t)N); }   // a 64-bit division is ten times the work
+        else { m = i / N; n = (int)(i % N); }
+        float* d = D + m * ldd + n;
         float o = alpha * (float)acc;
         if (beta != 0.f) o += beta * *d;
         if (bias) o += bias[n];
@@ -663,30 +708,29 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
     }
 }
 
-// partial[z][co][(kh*kW+kw)*Cp + ci]  ->  dW[co][ci][kh][kw], Cp = Cin padded to whole 32-channel chunks.  Threads walk the SOURCE
-// order (coalesced reads of every split; walking the destination order reads with a stride of Cin floats, eight times the sectors),
-// eight splits are requested before the first one is added, and only the single write per element is scattered.
+// partial[z][co][(kh*kW+kw)*Cp + ci]  ->  dW[co][ci][kh][kw], Cp = Cin padded to whole 32-channel chunks.  A block owns 32 elements
+// and deals the planes to its eight warps in equal runs, added in order: reads are whole 128-byte lines of every plane, and a small
+// filter over hundreds of planes still fills the chip (64 -> 64 channels, 592 planes: one element per thread left 144 blocks, 50 us).
+// Only the single write per element is scattered.
 __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, const float* __restrict__ partial, int splits,
                                                         int Cout, int Cin, int Cp, int T) {
     ncc::pdl_wait();
-    const size_t total = (size_t)Cout * Cp * T, stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t src = (size_t)blockIdx.x * blockDim.x + threadIdx.x; src < total; src += stride) {
-        const int ci = (int)(src % Cp);
-        if (ci >= Cin) continue;
-        double acc = 0.0;
-        int z = 0;
-        for (; z + 8 <= splits; z += 8) {
-            float v[8];
+    __shared__ double part[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t total = (size_t)Cout * Cp * T;   // a multiple of 32
+    const int per = (splits + 7) / 8, z0 = warp * per < splits ? warp * per : splits, zn = (splits - z0) < per ? (splits - z0) : per;
+    for (size_t base = blockIdx.x * (size_t)32; base < total; base += gridDim.x * (size_t)32) {
+        part[warp][lane] = sum_planes(partial + (size_t)z0 * total + base + lane, zn, total);
+        __syncthreads();
+        const size_t r = base / (unsigned)Cp, co = r / (unsigned)T;
+        const int ci = (int)(base - r * Cp) + lane, tap = (int)(r - co * T);
+        if (warp == 0 && ci < Cin) {
+            double acc = 0.0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = partial[(size_t)(z + k) * total + src];
-#pragma unroll
-            for (int k = 0; k < 8; k++) acc += (double)v[k];
+            for (int w = 0; w < 8; w++) acc += part[w][lane];
+            dW[(co * Cin + ci) * T + tap] = (float)acc;
         }
-        for (; z < splits; z++) acc += (double)partial[(size_t)z * total + src];
-        const size_t r = src / Cp;
-        const int tap = (int)(r % T);
-        const size_t co = r / T;
-        dW[(co * Cin + ci) * T + tap] = (float)acc;
+        __syncthreads();
     }
 }
 
@@ -714,17 +758,18 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(float* __restrict__ w
 // ------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------
-template <int BN, bool A_MN, bool B_MN, int NACC>
+template <int BN, bool A_MN, bool B_MN, bool SPLIT>
 static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p_in, dim3 tiles, cudaStream_t st) {
-    using Cfg = TileCfg<BN, NACC>;
+    using Cfg = TileCfg<BN, SPLIT>;
     TcParams p = p_in;
+    p.segment = SPLIT ? kSegment : 0x40000000;
     p.tiles_n = (int)tiles.x; p.tiles_m = (int)tiles.y; p.splits = (int)tiles.z;
     p.stages = Cfg::STAGES;
     const long long total = (long long)tiles.x * tiles.y * tiles.z;
     const int sms = ncc::sm_count();
     dim3 grid((unsigned)(total < sms ? total : sms), 1, 1);
     static bool attr_set = false;
-    auto kern = tc_kernel<BN, A_MN, B_MN, NACC>;
+    auto kern = tc_kernel<BN, A_MN, B_MN, SPLIT>;
     if (!attr_set) {
         NCC_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_set = true;
@@ -739,17 +784,17 @@ static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const TcPara
 
 template <bool A_MN, bool B_MN>
 static int launch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const TcParams& p, dim3 grid, cudaStream_t st) {
-    const bool two = p.kind == KIND_GEMM && p.passes == 3;   // two accumulators
+    const bool split = p.planes == 2;
     switch (bn) {
-        case 64: return two ? launch_one<64, A_MN, B_MN, 2>(ta, tb, p, grid, st) : launch_one<64, A_MN, B_MN, 1>(ta, tb, p, grid, st);
-        case 128: return two ? launch_one<128, A_MN, B_MN, 2>(ta, tb, p, grid, st) : launch_one<128, A_MN, B_MN, 1>(ta, tb, p, grid, st);
-        case 256: return launch_one<256, A_MN, B_MN, 1>(ta, tb, p, grid, st);
+        case 64: return split ? launch_one<64, A_MN, B_MN, true>(ta, tb, p, grid, st) : launch_one<64, A_MN, B_MN, false>(ta, tb, p, grid, st);
+        case 128: return split ? launch_one<128, A_MN, B_MN, true>(ta, tb, p, grid, st) : launch_one<128, A_MN, B_MN, false>(ta, tb, p, grid, st);
+        case 256: return launch_one<256, A_MN, B_MN, false>(ta, tb, p, grid, st);
     }
     return ncc::set_status(NC_CUDA_ERR_ARG, "tc: unsupported tile width %d", bn);
 }
 
-// two accumulators of a 3xTF32 product (and their double buffering) fit in tensor memory for up to 128 columns
-static int pick_bn(int N, bool two_acc = false) { return N <= 64 ? 64 : ((N <= 128 || two_acc) ? 128 : 256); }
+// sums kept in registers fit for up to 128 columns
+static int pick_bn(int N, bool split) { return N <= 64 ? 64 : ((N <= 128 || split) ? 128 : 256); }
 
 // splits over the reduction so that about one wave of CTAs exists; each split keeps >= 4 tiles
 static void pick_splits(int tiles, int nk, int* splits, int* kps) {
@@ -801,10 +846,9 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
     TcParams p = {};
     p.kind = KIND_GEMM;
     p.M = M; p.N = N;
-    p.passes = planes == 2 ? 3 : 1;
-    p.pass_tiles = (K + BK - 1) / BK;
+    p.planes = planes;
+    p.num_k_tiles = (K + BK - 1) / BK;
     p.a_plane = a_mn ? k_rows : M; p.b_plane = b_mn ? k_rows : N;
-    p.num_k_tiles = p.pass_tiles * p.passes;
     p.D = D; p.ldd = ldd; p.bias = bias; p.alpha = alpha; p.beta = beta;
     p.err = ncc::device_error_word();
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
@@ -859,7 +903,8 @@ static int convt_launch(float* y, int Hout, int Wout, int os, const float* xs, c
     int mh = 0, mw = 0;
     for (int i = 0; i < classes; i++) { mh = cls[i].Ho > mh ? cls[i].Ho : mh; mw = cls[i].Wo > mw ? cls[i].Wo : mw; }
     int bw = 1, bh = 1, bnn = 1;
-    pick_box(256, mw, mh, N, &bw, &bh, &bnn, 8, 256 / stride);
+    const int px = planes == 2 ? 128 : 256;   // pixels per tile: 3xTF32 keeps its sums in registers
+    pick_box(px, mw, mh, N, &bw, &bh, &bnn, 8, 256 / stride);
     CUtensorMap ta, tb;
     unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)wrows_total * planes};
     unsigned long long ws[1] = {(unsigned long long)Cin};
@@ -873,7 +918,7 @@ static int convt_launch(float* y, int Hout, int Wout, int os, const float* xs, c
     p.kind = KIND_CONVT;
     p.M = Cout;
     p.cchunks = (Cin + 31) / 32;
-    p.passes = planes == 2 ? 3 : 1;
+    p.planes = planes;
     p.a_plane = (int)wrows_total; p.b_plane = N;
     p.D = y; p.ldd = Cout; p.bias = bias; p.alpha = 1.f; p.beta = 0.f;
     p.bw = bw; p.bh = bh; p.bn = bnn;
@@ -892,14 +937,14 @@ static int convt_launch(float* y, int Hout, int Wout, int os, const float* xs, c
     }
     if (tiles_px > (1ll << 30)) return NC_CUDA_ERR_UNSUPPORTED;
     p.N = 0x7fffffff;
-    p.pass_tiles = p.k_tiles_per_split = p.num_k_tiles = 1;   // per class, see tile_of
+    p.k_tiles_per_split = p.num_k_tiles = 1;   // per class, see tile_of
     dim3 tiles((unsigned)tiles_px, (unsigned)((Cout + BM - 1) / BM), 1);
     p.flops = flops;
     // launch_one uses min(tiles, SMs) persistent CTAs: one statistics slab per CTA
     const long long total_tiles = (long long)tiles.x * tiles.y;
     const int n_ctas = (int)(total_tiles < ncc::sm_count() ? total_tiles : ncc::sm_count());
     if (want_stats) p.stat = ncc::conv_stats_buffer((size_t)n_ctas, Cout, st);
-    const int rc = launch_one<256, false, false, 1>(ta, tb, p, tiles, st);
+    const int rc = launch_bn<false, false>(px, ta, tb, p, tiles, st);
     if (rc == NC_CUDA_OK && p.stat) ncc::conv_stats_publish(y, Cout, (long long)N * Hout * Wout, n_ctas, p.stat);
     return rc;
 }
@@ -923,7 +968,7 @@ int conv_nhwc(float* y, const float* x, const float* wpacked, const float* bias,
         c.kH = kH; c.kW = kW; c.pad_h = c.pad_w = pad; c.Ho = Ho; c.Wo = Wo;
         return convt_launch(y, Ho, Wo, 1, xs, wpacked, (long long)kH * kW * Cout, bias, N, H, W, Cin, Cout, 1, &c, 1, mode, ncc::conv_stats_wanted(), flops, st);
     }
-    const int bn_cols = pick_bn(Cout);
+    const int bn_cols = pick_bn(Cout, planes == 2);
     int bw = 1, bh = 1, bnn = 1;
     pick_box(128, Wo, Ho, N, &bw, &bh, &bnn);
     CUtensorMap ta, tb;
@@ -941,10 +986,9 @@ int conv_nhwc(float* y, const float* x, const float* wpacked, const float* bias,
     p.kind = KIND_CONV;
     p.M = N * Ho * Wo; p.N = Cout;
     p.cchunks = (Cin + 31) / 32;
-    p.passes = planes == 2 ? 3 : 1;
-    p.pass_tiles = kH * kW * p.cchunks;
+    p.planes = planes;
     p.a_plane = N; p.b_plane = kH * kW * Cout;
-    p.num_k_tiles = p.pass_tiles * p.passes;
+    p.num_k_tiles = kH * kW * p.cchunks;
     p.k_tiles_per_split = p.num_k_tiles;
     p.D = y; p.ldd = Cout; p.bias = bias; p.alpha = 1.f; p.beta = 0.f;
     p.bw = bw; p.bh = bh; p.bn = bnn;
@@ -1023,8 +1067,8 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
     const int Ncols = kH * kW * Cp;
     // column tile: whole filter rows when they fit in 256 columns, else 256 / 128 / 64
     int bn_cols;
-    if (kW * Cp == 64 || kW * Cp == 128 || kW * Cp == 192 || kW * Cp == 256) bn_cols = kW * Cp;
-    else bn_cols = pick_bn(Ncols);
+    if (planes == 1 && (kW * Cp == 64 || kW * Cp == 128 || kW * Cp == 192 || kW * Cp == 256)) bn_cols = kW * Cp;
+    else bn_cols = pick_bn(Ncols, planes == 2);
     int bw = 1, bh = 1, bnn = 1;
     // split operands: a box that hung over the last image of the hi plane would read the lo plane instead of zeros
     pick_box(32, Wo, Ho, N, &bw, &bh, &bnn, 1, 256 / stride, planes == 2);
@@ -1045,10 +1089,9 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
     p.tiles_w = (Wo + bw - 1) / bw; p.tiles_h = (Ho + bh - 1) / bh;
     p.Ho = Ho; p.Wo = Wo; p.Nimg = N;
     p.kW = kW; p.pad = pad; p.stride = stride; p.Cin = Cp;
-    p.passes = planes == 2 ? 3 : 1;
-    p.pass_tiles = p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
+    p.planes = planes;
+    p.num_k_tiles = p.tiles_w * p.tiles_h * ((N + bnn - 1) / bnn);
     p.a_plane = p.b_plane = N;
-    p.num_k_tiles = p.pass_tiles * p.passes;
     p.alpha = 1.f;
     p.err = ncc::device_error_word();
     const int tiles_m = (Cout + BM - 1) / BM, tiles_n = (Ncols + bn_cols - 1) / bn_cols;
@@ -1060,7 +1103,7 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
     dim3 grid(tiles_n, tiles_m, splits);
     p.flops = 2.0 * N * Ho * Wo * (double)Cout * Cin * kH * kW;
     int rc;
-    if (bn_cols == 192) rc = launch_one<192, true, true, 1>(ta, tb, p, grid, st);
+    if (bn_cols == 192) rc = launch_one<192, true, true, false>(ta, tb, p, grid, st);
     else rc = launch_bn<true, true>(bn_cols, ta, tb, p, grid, st);
     if (rc) return rc;
     return dw_reduce(dW, p.partial, splits, Cout, Cin, kH, kW, st);
@@ -1068,7 +1111,7 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
 
 int dw_reduce(float* dW, const float* partial, int splits, int Cout, int Cin, int kH, int kW, cudaStream_t st) {
     const int Cp = (Cin + 31) & ~31;
-    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cp * kH * kW, 256), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
+    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cp * kH * kW / 32, 1), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("dw_reduce");
 }
