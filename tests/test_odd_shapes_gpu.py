@@ -32,6 +32,7 @@ CONV = [
     (1, 36, 70, 66, 100, 3, 1, 1),
     (5, 192, 11, 11, 192, 3, 1, 1),  # low images: per-tap kernel
     (3, 40, 11, 13, 24, 3, 1, 1),
+    (2, 32, 14, 15, 32, 9, 1, 4),    # more than 64 taps
 ]
 
 
@@ -81,3 +82,22 @@ def test_linear_odd(abi, mode, tol, B, I, Oo):  # noqa: F811
     close(host(gx), dx, tol)
     close(host(gW), dW, tol)
     close(host(gb), db, TOL_F32)
+
+
+# products that fill the chip without a split reduction: 256 x 256 tiles of SM pairs with remainders in rows, columns (also ones whose
+# output rows are no whole 16-byte pieces) and reduction, one tile and several per pair, every operand order, alpha and beta
+@pytest.mark.parametrize("M,N,K,ta,tb", [(2561, 1024, 160, 0, 1), (2500, 1030, 196, 0, 1), (2080, 1056, 132, 1, 0), (2464, 1088, 1000, 0, 0),
+                                         (1056, 2500, 256, 1, 1), (4999, 2052, 128, 0, 1)])
+def test_large_products(abi, M, N, K, ta, tb):  # noqa: F811
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((K, M) if ta else (M, K)).astype(np.float32), rng.standard_normal((N, K) if tb else (K, N)).astype(np.float32)
+    C, b = rng.standard_normal((M, N)).astype(np.float32), rng.standard_normal(N).astype(np.float32)
+    prod = (A.T if ta else A).astype(np.float64) @ (B.T if tb else B).astype(np.float64)
+    for mode, tol in MODES:
+        abi.nc_cuda_set_math_mode(mode)
+        plain, full = torch.full((M, N), float("nan"), device="cuda"), dev(C)
+        for out, alpha, beta, bias in ((plain, 1.0, 0.0, None), (full, 0.5, -2.0, b)):
+            ok(abi, abi.nc_cuda_matmul_f32_ex(P(out), N, P(dev(A)), A.shape[1], P(dev(B)), B.shape[1], M, N, K, alpha, beta, ta, tb,
+                                              P(dev(bias)) if bias is not None else None, None))
+        close(host(plain), prod, tol)
+        close(host(full), 0.5 * prod - 2.0 * C + b, tol)

@@ -78,6 +78,23 @@ def test_small_conv(abi, layout, N, Ci, H, W, Co, k, p):  # noqa: F811
         close(host(gb), dbo, TOL_F32)
 
 
+def test_small_conv_infinity(abi):  # noqa: F811
+    """An infinity in the last input column reaches the weight gradient's last filter column only, also beside the padding of a row
+    group of four (seven output columns)."""
+    from nocta_b200.cuda_abi import size4
+    H = W = 9
+    x, g = np.ones((1, 1, H, W), np.float32), np.ones((1, 2, 7, 7), np.float32)
+    x[0, 0, 0, 8] = np.inf
+    abi.nc_cuda_set_math_mode(MODE_TF32)
+    gw = torch.zeros(18, device="cuda")
+    ok(abi, abi.nc_cuda_conv2d_backward_weight_f32_ex(P(gw), None, P(dev(g)), size4([98, 49, 7, 1]), P(dev(x)), size4([81, 81, 9, 1]),
+                                                      1, 1, H, W, 2, 3, 3, 1, 0, None))
+    got = host(gw).reshape(2, 3, 3)
+    assert np.isposinf(got[:, 0, 2]).all()
+    got[:, 0, 2] = 49.0
+    assert (got == 49.0).all()
+
+
 # rows x columns: a row per block and a row per warp (2368 rows and more), vector and scalar columns, the most columns a block's
 # registers hold, and more than that
 @pytest.mark.parametrize("rows,cols", [(1, 1), (3, 31), (16, 1024), (2, 8192), (2, 8196), (5, 1025), (2400, 64), (2400, 310), (2500, 1024), (2500, 1028)])
