@@ -816,6 +816,16 @@ bool gemm_eligible(int M, int N, int K, bool aligned) {
     return M >= 32 && N >= 16 && K >= 32 && (long long)M * N * K >= (aligned ? 1ll << 22 : 1ll << 24);
 }
 
+// Whether a product that fills the chip without splitting its reduction runs on pairs of SMs (tc_gemm2.cu): as long as tiles twice the
+// height take no more waves.  Residual MLP step at batch 4096 (24 products of 34 GFLOP) 2350 -> 2196 us, 500 -> 560 TFLOP/s a product;
+// the sustained TF32 rate of the chip, half of bf16's, is 683.
+static bool pair_wins(int M, int N, int K) {
+    const long long sms = ncc::sm_count();
+    const long long one = ((M + BM - 1) / BM) * (long long)((N + 255) / 256), two = ((M + 255) / 256) * (long long)((N + 255) / 256);
+    const long long waves1 = (one + sms - 1) / sms, waves2 = (two + sms / 2 - 1) / (sms / 2);
+    return N > 128 && M > 128 && K >= 128 && waves2 <= waves1;
+}
+
 int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N, int K,
          const float* bias, float alpha, float beta, int mode, cudaStream_t st) {
     const bool a_ok = !(lda & 3) && !(reinterpret_cast<uintptr_t>(A) & 15u), b_ok = !(ldb & 3) && !(reinterpret_cast<uintptr_t>(B) & 15u);
@@ -854,6 +864,10 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
     int splits, kps;
     pick_splits(tiles_m * tiles_n, p.num_k_tiles, &splits, &kps);
+    if (planes == 1 && splits == 1 && pair_wins(M, N, K)) {
+        const int rc = gemm_pair(D, ldd, A, lda, a_mn, B, ldb, b_mn, M, N, K, bias, alpha, beta, st);
+        if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
+    }
     p.k_tiles_per_split = kps;
     if (splits > 1) {
         p.partial = (float*)ncc::scratch(2, sizeof(float) * (size_t)splits * M * N, st);

@@ -14,6 +14,11 @@ namespace tc {
 int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N,
          int K, const float* bias, float alpha, float beta, int mode, cudaStream_t st);
 
+// The same in plain TF32 on pairs of SMs (tc_gemm2.cu), 256 x 256 tiles, no split; operands TMA can describe, an MN-major operand's
+// extent a multiple of 32; NC_CUDA_ERR_UNSUPPORTED otherwise.
+int gemm_pair(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N, int K,
+              const float* bias, float alpha, float beta, cudaStream_t st);
+
 // whether gemm() takes a product of these sizes; aligned: both operands are made of 16-byte pieces
 bool gemm_eligible(int M, int N, int K, bool aligned);
 
