@@ -159,6 +159,15 @@ static void accumulate_leaf(nc_tensor* leaf, nc_tensor* g) {
                 return;
             }
         }
+        if (!g->is_contiguous && g->dtype == leaf->dtype && g->storage->device == leaf->storage->device && nc_tensor_shape_eq(g, leaf)) {
+            /* another order in memory (a convolution's input gradient is channels-last): one copy in the leaf's order */
+            leaf->grad = nc_tensor_contiguous(g);
+            if (!leaf->grad) return;
+            leaf->grad->is_leaf = true;
+            leaf->grad->is_reachable = true;
+            if (g_ready_fn) g_ready_fn(leaf, g_ready_ctx);
+            return;
+        }
         leaf->grad = nci_empty_on(leaf->shape, leaf->ndim, leaf->dtype, leaf->storage->device);
         if (!leaf->grad) return;
         nc_tensor_fill_(leaf->grad, 0.0);
