@@ -708,29 +708,36 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(float* __restrict__ 
     }
 }
 
-// partial[z][co][(kh*kW+kw)*Cp + ci]  ->  dW[co][ci][kh][kw], Cp = Cin padded to whole 32-channel chunks.  A block owns 32 elements
-// and deals the planes to its eight warps in equal runs, added in order: reads are whole 128-byte lines of every plane, and a small
-// filter over hundreds of planes still fills the chip (64 -> 64 channels, 592 planes: one element per thread left 144 blocks, 50 us).
-// Only the single write per element is scattered.
+// partial[z][co][(kh*kW+kw)*Cp + ci]  ->  dW[co][ci][kh][kw], Cp = Cin padded to whole 32-channel chunks.  A warp takes 32 elements of
+// one run of planes, so reads are whole 128-byte lines of every plane; G warps share the planes of their elements in equal runs, added
+// in order.  G = 8 from 64 planes on, where few weights leave the chip idle otherwise (64 -> 64 channels, 592 planes: one element per
+// thread left 144 blocks, 50 us); with fewer planes a warp has too little to do between the barriers (256 -> 256 channels, 12 planes:
+// 20 us with eight warps, 9 with one).  Only the single write per element is scattered.
+template <int G>
 __global__ void __launch_bounds__(256) dw_reduce_kernel(float* __restrict__ dW, const float* __restrict__ partial, int splits,
                                                         int Cout, int Cin, int Cp, int T) {
     ncc::pdl_wait();
-    __shared__ double part[8][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double part[G][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp % G;
     const size_t total = (size_t)Cout * Cp * T;   // a multiple of 32
-    const int per = (splits + 7) / 8, z0 = warp * per < splits ? warp * per : splits, zn = (splits - z0) < per ? (splits - z0) : per;
-    for (size_t base = blockIdx.x * (size_t)32; base < total; base += gridDim.x * (size_t)32) {
-        part[warp][lane] = sum_planes(partial + (size_t)z0 * total + base + lane, zn, total);
-        __syncthreads();
-        const size_t r = base / (unsigned)Cp, co = r / (unsigned)T;
-        const int ci = (int)(base - r * Cp) + lane, tap = (int)(r - co * T);
-        if (warp == 0 && ci < Cin) {
-            double acc = 0.0;
+    const int per = (splits + G - 1) / G, z0 = g * per < splits ? g * per : splits, zn = (splits - z0) < per ? (splits - z0) : per;
+    constexpr size_t kBlock = 32 * 8 / G;         // elements of a block
+    for (size_t base = blockIdx.x * kBlock; base < total; base += gridDim.x * kBlock) {
+        const size_t at = base + (size_t)(warp / G) * 32;
+        double acc = at < total ? sum_planes(partial + (size_t)z0 * total + at + lane, zn, total) : 0.0;
+        if (G > 1) {
+            part[g][lane] = acc;
+            __syncthreads();
+            if (g == 0) {
+                acc = 0.0;
 #pragma unroll
-            for (int w = 0; w < 8; w++) acc += part[w][lane];
-            dW[(co * Cin + ci) * T + tap] = (float)acc;
+                for (int w = 0; w < G; w++) acc += part[w][lane];
+            }
         }
-        __syncthreads();
+        const size_t r = at / (unsigned)Cp, co = r / (unsigned)T;
+        const int ci = (int)(at - r * Cp) + lane, tap = (int)(r - co * T);
+        if (g == 0 && at < total && ci < Cin) dW[(co * Cin + ci) * T + tap] = (float)acc;
+        if (G > 1) __syncthreads();
     }
 }
 
@@ -810,6 +817,34 @@ static void pick_splits(int tiles, int nk, int* splits, int* kps) {
     *splits = (nk + per - 1) / per;
 }
 
+// cycles of one reduction tile with bn columns: four k-steps of MMA (max(N / 2, operand bytes / 128, 46) cycles each, three of them for
+// split operands), or its loads at the 70 bytes per cycle that an SM gets of L2 when all of them load
+static double tile_cycles(int bn, int planes) {
+    const double mma = 4.0 * (bn / 2 > (BM + bn) / 4 ? bn / 2 : ((BM + bn) / 4 > 46 ? (BM + bn) / 4 : 46)) * (planes == 2 ? 3 : 1);
+    const double load = (BM + bn) * 128.0 * planes / 70.0;
+    return mma > load ? mma : load;
+}
+// Columns per tile and splits of a product.  Wide tiles split until about one wave of CTAs exists are right where the reduction is
+// long; otherwise the second kernel of a split costs more (about 5000 cycles and the partial sums' traffic) than narrower tiles lose.
+// They are taken where the estimate is at least 15 % lower: 1001 x 1250 outputs, K = 310: two splits of 40 tiles -> 80 tiles of 128
+// columns; 1001 x 310, K = 1250: nine splits -> three of 64 columns.
+static void pick_tile(int M, int N, int nk, int planes, int* bn, int* splits, int* kps) {
+    const int sms = ncc::sm_count(), rows = (M + BM - 1) / BM;
+    auto cost = [&](int b, int s, int per) {
+        const long long ctas = (long long)rows * ((N + b - 1) / b) * s, waves = (ctas + sms - 1) / sms;
+        return (double)waves * (per * tile_cycles(b, planes) + 600.0) + 2000.0 + 8.0 * b + (s > 1 ? 5000.0 + (double)s * M * N * 8.0 / 3500.0 : 0.0);
+    };
+    *bn = pick_bn(N, planes == 2);
+    pick_splits(rows * ((N + *bn - 1) / *bn), nk, splits, kps);
+    double best = 0.85 * cost(*bn, *splits, *kps);
+    for (int b = *bn; b >= 64; b /= 2) {
+        int s, per;
+        pick_splits(rows * ((N + b - 1) / b), nk, &s, &per);
+        if (cost(b, s, per) < best) { best = cost(b, s, per); *bn = b; *splits = s; *kps = per; }
+        if (s > 1 && cost(b, 1, nk) < best) { best = cost(b, 1, nk); *bn = b; *splits = 1; *kps = nk; }
+    }
+}
+
 // Rows beyond M inside the 128-row tile are zero-filled by TMA and never stored; small products stay on CUDA cores.  Operands whose
 // rows are no whole 16-byte pieces cost a copy each first: from 2^24 multiply-adds on.
 bool gemm_eligible(int M, int N, int K, bool aligned) {
@@ -823,7 +858,7 @@ static bool pair_wins(int M, int N, int K) {
     const long long sms = ncc::sm_count();
     const long long one = ((M + BM - 1) / BM) * (long long)((N + 255) / 256), two = ((M + 255) / 256) * (long long)((N + 255) / 256);
     const long long waves1 = (one + sms - 1) / sms, waves2 = (two + sms / 2 - 1) / (sms / 2);
-    return N > 128 && M > 128 && K >= 128 && waves2 <= waves1;
+    return K >= 128 && waves2 <= waves1;
 }
 
 int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, int ldb, bool b_mn, int M, int N, int K,
@@ -841,7 +876,8 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
         return true;
     };
     if (!prepare(kSlotA, A, lda, a_mn, M, a_ok) || !prepare(kSlotB, B, ldb, b_mn, N, b_ok)) return NC_CUDA_ERR_RUNTIME;
-    const int bn = pick_bn(N, planes == 2);
+    int bn, splits, kps;
+    pick_tile(M, N, (K + BK - 1) / BK, planes, &bn, &splits, &kps);
     CUtensorMap ta, tb;
     {
         unsigned long long dims[2], str[1];
@@ -862,9 +898,7 @@ int gemm(float* D, int ldd, const float* A, int lda, bool a_mn, const float* B, 
     p.D = D; p.ldd = ldd; p.bias = bias; p.alpha = alpha; p.beta = beta;
     p.err = ncc::device_error_word();
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
-    int splits, kps;
-    pick_splits(tiles_m * tiles_n, p.num_k_tiles, &splits, &kps);
-    if (planes == 1 && splits == 1 && pair_wins(M, N, K)) {
+    if (planes == 1 && splits == 1 && bn == 256 && pair_wins(M, N, K)) {
         const int rc = gemm_pair(D, ldd, A, lda, a_mn, B, ldb, b_mn, M, N, K, bias, alpha, beta, st);
         if (rc != NC_CUDA_ERR_UNSUPPORTED) return rc;
     }
@@ -917,7 +951,16 @@ static int convt_launch(float* y, int Hout, int Wout, int os, const float* xs, c
     int mh = 0, mw = 0;
     for (int i = 0; i < classes; i++) { mh = cls[i].Ho > mh ? cls[i].Ho : mh; mw = cls[i].Wo > mw ? cls[i].Wo : mw; }
     int bw = 1, bh = 1, bnn = 1;
-    const int px = planes == 2 ? 128 : 256;   // pixels per tile: 3xTF32 keeps its sums in registers
+    // Pixels per tile: 128 where twice the tiles are done sooner, as for the low images at the end of a network (37 images of 22 x 22:
+    // 60 tiles of 256 on 148 SMs, 27 us), else 256, but for 3xTF32, which keeps its sums in registers.
+    auto waves = [&](int px) {
+        pick_box(px, mw, mh, N, &bw, &bh, &bnn, 8, 256 / stride);
+        long long t = 0;
+        for (int i = 0; i < classes; i++) t += (long long)((cls[i].Wo + bw - 1) / bw) * ((cls[i].Ho + bh - 1) / bh) * ((N + bnn - 1) / bnn);
+        t *= (Cout + BM - 1) / BM;
+        return (double)((t + ncc::sm_count() - 1) / ncc::sm_count());
+    };
+    const int px = planes == 2 || waves(128) * tile_cycles(128, 1) < waves(256) * tile_cycles(256, 1) ? 128 : 256;
     pick_box(px, mw, mh, N, &bw, &bh, &bnn, 8, 256 / stride);
     CUtensorMap ta, tb;
     unsigned long long wd[2] = {(unsigned long long)Cin, (unsigned long long)wrows_total * planes};
@@ -1125,7 +1168,9 @@ int conv_dw_nhwc(float* dW, const float* dy, const float* x, int N, int H, int W
 
 int dw_reduce(float* dW, const float* partial, int splits, int Cout, int Cin, int kH, int kW, cudaStream_t st) {
     const int Cp = (Cin + 31) & ~31;
-    ncc::launch(dw_reduce_kernel, ncc::grid_for((long long)Cout * Cp * kH * kW / 32, 1), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
+    const long long total = (long long)Cout * Cp * kH * kW;
+    if (splits >= 64) ncc::launch(dw_reduce_kernel<8>, ncc::grid_for(total / 32, 1), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
+    else ncc::launch(dw_reduce_kernel<1>, ncc::grid_for(total, 256), 256, 0, st, dW, partial, splits, Cout, Cin, Cp, kH * kW);
     NCC_COUNT_LAUNCH();
     return ncc::launch_status("dw_reduce");
 }
