@@ -2,8 +2,8 @@
 // the output (forward) or reading the output gradient (weight gradient), not by arithmetic.
 // TF32 mode with 64 output channels: tensor-core kernels (namespaces tcf and tcw below) whose operand rows are the 27-wide
 // patches padded to 32 floats, built in shared memory by the threads themselves.
-// Other modes and channel counts: CUDA-core kernels.  Forward: a shared-memory tiled kernel for the common channel counts,
-// else 4..16 threads per output pixel, 16 output channels each, the 27 patch values in registers.  Weight gradient: the
+// Other modes and channel counts: CUDA-core kernels.  Forward: a shared-memory tiled kernel up to 128 channels,
+// else 9..16 threads per output pixel, 16 output channels each, the 27 patch values in registers.  Weight gradient: the
 // reduction over all pixels is split over CTAs; each CTA stages 64-pixel tiles of dY and of the 27-wide patches in shared
 // memory (see dw_tile_kernel); per-CTA partial sums are combined in a fixed order.  No input gradient: the network input
 // needs none.
@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(256) fwd_kernel(float* __restrict__ y, const f
     }
 }
 
-// Tiled forward for Cout in {16, 32, 64, 128}.  A CTA owns a strip of TR output rows x 64 output columns
+// Tiled forward for up to 128 channels: COUT is g.Cout rounded up to 16, 32, 64 or 128, channels beyond g.Cout have zero weights
+// and are not stored (48 channels, 37 images of 44 x 44: 38 us with the kernel above, 18 us with this one).  A CTA owns a strip of TR output rows x 64 output columns
 // of one image: the 3 x (TR+2) x 66 input halo is staged in shared memory once (coalesced reads, zero
 // fill = padding), every thread computes 4 consecutive pixels x 8 output channels (channels cg*4..+3 and
 // Cout/2 + cg*4..+3, so that the lanes of a warp store whole 128-byte lines), reading its 6 input
@@ -105,9 +106,9 @@ __global__ void __launch_bounds__(256, 4) fwd_tile_kernel(float* __restrict__ y,
     __shared__ __align__(16) float tile[3][ROWS][TWP];
     for (int i = threadIdx.x; i < K * COUT; i += 256) {
         const int co = i % COUT, k = i / COUT;
-        ws[i] = w[co * K + k];
+        ws[i] = co < g.Cout ? w[co * K + k] : 0.f;
     }
-    for (int i = threadIdx.x; i < COUT; i += 256) bs[i] = bias ? bias[i] : 0.f;
+    for (int i = threadIdx.x; i < COUT; i += 256) bs[i] = bias && i < g.Cout ? bias[i] : 0.f;
     // per-channel sum and sum of squares of this CTA's outputs, one private row per warp (no atomics: the result
     // does not depend on the order in which warps run)
     __shared__ float ssum[STAT ? 8 : 1][STAT ? 2 * COUT : 1];
@@ -169,12 +170,13 @@ __global__ void __launch_bounds__(256, 4) fwd_tile_kernel(float* __restrict__ y,
             }
         const int ho = ho0 + prow;
         if (ho < g.Ho) {
-            float* dst = y + ((size_t)(n * g.Ho + ho) * g.Wo + wo0 + pcol) * COUT;
+            float* dst = y + ((size_t)(n * g.Ho + ho) * g.Wo + wo0 + pcol) * g.Cout;
 #pragma unroll
             for (int p = 0; p < 4; p++) {
-                if (wo0 + pcol + p < g.Wo) {
-                    *reinterpret_cast<float4*>(dst + (size_t)p * COUT + cg * 4) = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
-                    *reinterpret_cast<float4*>(dst + (size_t)p * COUT + COUT / 2 + cg * 4) = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
+                if (wo0 + pcol + p < g.Wo) {   // more than half of the padded channels exist, in multiples of four
+                    *reinterpret_cast<float4*>(dst + p * g.Cout + cg * 4) = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+                    if (COUT / 2 + cg * 4 < g.Cout)
+                        *reinterpret_cast<float4*>(dst + p * g.Cout + COUT / 2 + cg * 4) = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
                 }
             }
         }
@@ -208,8 +210,8 @@ __global__ void __launch_bounds__(256, 4) fwd_tile_kernel(float* __restrict__ y,
     }
     if (STAT) {
         __syncthreads();
-        for (int i = threadIdx.x; i < COUT; i += 256) {
-            double* sd = stat + ((size_t)blockIdx.x * COUT + i) * 2;
+        for (int i = threadIdx.x; i < g.Cout; i += 256) {
+            double* sd = stat + ((size_t)blockIdx.x * g.Cout + i) * 2;
             double a = 0.0, b = 0.0;
 #pragma unroll
             for (int wp = 0; wp < 8; wp++) {
@@ -229,7 +231,7 @@ static int launch_fwd_tile(float* y, const float* x, const float* w, const float
     const long long cap = (long long)ncc::sm_count() * 4;  // 4 CTAs of 64 registers x 256 threads fit an SM
     const int grid = (int)(ntiles < cap ? ntiles : cap);
     // a BatchNorm that follows can take the per-channel sums from here instead of reading y again (one slab per CTA)
-    double* stat = ncc::conv_stats_wanted() ? ncc::conv_stats_buffer((size_t)grid, COUT, st) : nullptr;
+    double* stat = g.Cout == COUT && ncc::conv_stats_wanted() ? ncc::conv_stats_buffer((size_t)grid, g.Cout, st) : nullptr;
     if (stat) {
         ncc::launch(fwd_tile_kernel<COUT, true>, grid, 256, 0, st, y, x, w, bias, g, tiles_h, tiles_w, (int)ntiles, stat);
     } else {
@@ -239,7 +241,8 @@ static int launch_fwd_tile(float* y, const float* x, const float* w, const float
     return grid;
 }
 
-// Tiled weight gradient for Cout in {32, 64}.  A CTA walks strips of 4 output rows x 64 columns; the
+// Tiled weight gradient.  A block takes COUT = 32 or 64 channels from blockIdx.y * COUT on, those beyond g.Cout by idle lanes (48
+// channels, 37 images of 44 x 44: 102 us on the general path, 31 us here).  A CTA walks strips of 4 output rows x 64 columns; the
 // input halo of a strip is staged in shared memory, dY is read straight from global memory (every
 // element is needed by exactly one thread; a warp reads whole 128/256-byte pixel rows).  A warp takes
 // groups of 4 consecutive pixels; lane l owns output channels l*CPT..+CPT-1 and ALL 27 taps, so the six
@@ -251,6 +254,8 @@ __global__ void __launch_bounds__(256) dw_tile_kernel(float* __restrict__ partia
                                                       const float* __restrict__ in, Geo g, int tiles_h, int tiles_w, int ntiles) {
     ncc::pdl_wait();
     constexpr int CPT = COUT / 32, TR = 4, ROWS = TR + 2, RS = (K * CPT) | 1;
+    const int co0 = blockIdx.y * COUT;
+    const bool live = co0 + (threadIdx.x & 31) * CPT < g.Cout;   // g.Cout is even: all or none of a lane's channels
     __shared__ __align__(16) float tile[3][ROWS][TWP];
     __shared__ float red[32][RS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -281,16 +286,16 @@ __global__ void __launch_bounds__(256) dw_tile_kernel(float* __restrict__ partia
             const int prow = grp / (TW / 4), pcol = (grp % (TW / 4)) * 4;
             const int ho = ho0 + prow;
             if (ho >= g.Ho || wo0 + pcol >= g.Wo) continue;  // warp-uniform
-            const float* src = dy + ((size_t)(n * g.Ho + ho) * g.Wo + wo0 + pcol) * COUT + lane * CPT;
+            const float* src = dy + ((size_t)(n * g.Ho + ho) * g.Wo + wo0 + pcol) * g.Cout + co0 + lane * CPT;
             float d[4][CPT];
 #pragma unroll
             for (int p = 0; p < 4; p++) {
-                const bool ok = wo0 + pcol + p < g.Wo;
+                const bool ok = live && wo0 + pcol + p < g.Wo;
                 if (CPT == 2) {
-                    float2 v = ok ? *reinterpret_cast<const float2*>(src + (size_t)p * COUT) : make_float2(0.f, 0.f);
+                    float2 v = ok ? *reinterpret_cast<const float2*>(src + p * g.Cout) : make_float2(0.f, 0.f);
                     d[p][0] = v.x; d[p][CPT - 1] = v.y;
                 } else {
-                    d[p][0] = ok ? src[(size_t)p * COUT] : 0.f;
+                    d[p][0] = ok ? src[p * g.Cout] : 0.f;
                 }
             }
 #pragma unroll
@@ -327,7 +332,7 @@ __global__ void __launch_bounds__(256) dw_tile_kernel(float* __restrict__ partia
     __syncthreads();
     for (int i = threadIdx.x; i < COUT * K; i += 256) {
         const int co = i / K, k = i % K;
-        partial[((size_t)blockIdx.x * COUT + co) * KP + k] = red[co / CPT][(co % CPT) * K + k];
+        if (co0 + co < g.Cout) partial[((size_t)blockIdx.x * g.Cout + co0 + co) * KP + k] = red[co / CPT][(co % CPT) * K + k];
     }
 }
 
@@ -737,12 +742,12 @@ int forward(float* y, const float* x, const long long xs[4], const float* w, con
     if (!fits_int(N, H, W, xs, g.Ho, g.Wo)) return NC_CUDA_ERR_UNSUPPORTED;
     const int pixels = N * g.Ho * g.Wo;
     if (Cout == tcf::COUT && ncc::math_mode() == NC_CUDA_MATH_TF32) return forward_tc(y, x, w, bias, g, st);
-    if (Cout == 16 || Cout == 32 || Cout == 64 || Cout == 128) {
+    if (Cout <= 128) {
         double* stat = nullptr;
         int slabs;
         if (Cout == 16) slabs = launch_fwd_tile<16>(y, x, w, bias, g, st, &stat);
         else if (Cout == 32) slabs = launch_fwd_tile<32>(y, x, w, bias, g, st, &stat);
-        else if (Cout == 64) slabs = launch_fwd_tile<64>(y, x, w, bias, g, st, &stat);
+        else if (Cout <= 64) slabs = launch_fwd_tile<64>(y, x, w, bias, g, st, &stat);
         else slabs = launch_fwd_tile<128>(y, x, w, bias, g, st, &stat);
         NCC_COUNT_LAUNCH();
         const int rc = ncc::launch_status("conv_first forward");
@@ -760,7 +765,6 @@ int forward(float* y, const float* x, const long long xs[4], const float* w, con
 }
 
 int weight_grad(float* dW, const float* dy, const float* x, const long long xs[4], int N, int H, int W, int Cout, int pad, cudaStream_t st) {
-    if (Cout != 64 && Cout != 32) return NC_CUDA_ERR_UNSUPPORTED;
     Geo g{N, H, W, Cout, pad, H + 2 * pad - 2, W + 2 * pad - 2, {(int)xs[0], (int)xs[1], (int)xs[2], (int)xs[3]}};
     if (g.Ho <= 0 || g.Wo <= 0) return NC_CUDA_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(dy) & 15u) != 0) return NC_CUDA_ERR_UNSUPPORTED;
@@ -776,7 +780,7 @@ int weight_grad(float* dW, const float* dy, const float* x, const long long xs[4
     if (blocks > ntiles) blocks = ntiles;
     float* partial = (float*)ncc::scratch(2, sizeof(float) * (size_t)blocks * Cout * KP, st);
     if (!partial) return NC_CUDA_ERR_RUNTIME;
-    if (Cout == 64) ncc::launch(dw_tile_kernel<64>, (int)blocks, 256, 0, st, partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
+    if (Cout > 32) ncc::launch(dw_tile_kernel<64>, dim3((unsigned)blocks, (unsigned)((Cout + 63) / 64)), 256, 0, st, partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
     else ncc::launch(dw_tile_kernel<32>, (int)blocks, 256, 0, st, partial, dy, x, g, tiles_h, tiles_w, (int)ntiles);
     NCC_COUNT_LAUNCH();
     ncc::launch(dw_reduce_kernel, ncc::ceil_div(Cout * K * 32, 256), 256, 0, st, dW, partial, (int)blocks, Cout);

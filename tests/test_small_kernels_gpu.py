@@ -129,3 +129,23 @@ def test_mse_sizes(abi, n):  # noqa: F811
         d = p.astype(np.float64) - t
         close(host(loss), np.array([(d * d).mean()]), TOL_F32)
         close(host(gp), 2.0 * d / n, TOL_F32)
+
+
+# first layer (3 input channels): channel counts that fill 32, 64 or 128 padded channels only in part, more than one group of 64, more
+# than the tiled forward kernel takes; image widths around the 64-pixel strip
+@pytest.mark.parametrize("N,H,W,Co", [(2, 9, 70, 48), (3, 5, 64, 16), (1, 12, 13, 80), (2, 7, 65, 112), (2, 6, 6, 176), (5, 10, 3, 96)])
+def test_first_layer_channels(abi, N, H, W, Co):  # noqa: F811
+    from nocta_b200.cuda_abi import size4
+    rng = np.random.default_rng(N + H + W + Co)
+    x, w, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, 3, H, W), (Co, 3, 3, 3), (Co,)))
+    g = rng.standard_normal((N, Co, H, W)).astype(np.float32)
+    _, dwo, dbo = O.conv2d_backward(x, w, g, 1, 1)
+    abi.nc_cuda_set_math_mode(MODE_TF32)
+    xs, ys = size4([3 * H * W, H * W, W, 1]), size4([H * W * Co, 1, W * Co, Co])
+    nan = lambda n: torch.full((n,), float("nan"), device="cuda")  # noqa: E731
+    y, gw, gb, tx, tg = nan(g.size), nan(w.size), nan(Co), dev(x), dev(g.transpose(0, 2, 3, 1))
+    ok(abi, abi.nc_cuda_conv2d_forward_f32_ex(P(y), ys, P(tx), xs, P(dev(w)), P(dev(b)), N, 3, H, W, Co, 3, 3, 1, 1, None))
+    ok(abi, abi.nc_cuda_conv2d_backward_weight_f32_ex(P(gw), P(gb), P(tg), ys, P(tx), xs, N, 3, H, W, Co, 3, 3, 1, 1, None))
+    close(host(y).reshape(N, H, W, Co).transpose(0, 3, 1, 2), O.conv2d_forward(x, w, b, 1, 1), TOL_F32)
+    close(host(gw).reshape(w.shape), dwo, TOL_F32)
+    close(host(gb), dbo, TOL_F32)
