@@ -36,36 +36,45 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(float* __restrict__ d
     constexpr int MR = MT * KS / kWarps;           // rows a warp sums
     static_assert(MR >= 1, "a row per warp");
     __shared__ float red[KS][MT][32];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar[2];
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, chunk = KS * slice, ks = warp % KS, r0 = warp / KS * MR;
     const int n = blockIdx.x / blocks_k * 32 + lane, m0 = blockIdx.y * MT;
     const int k0 = (int)(blockIdx.x % blocks_k) * chunk, kb = (K - k0) < chunk ? (K - k0) : chunk;   // this block's k
-    const int kn = (kb - ks * slice) < slice ? (kb - ks * slice) : slice;                            // this warp's; may be <= 0
     float* xs = sm;
     float* ws = sm + MT * chunk;
     if (threadIdx.x == 0) {
-        tc::mbar_init(tc::smem_u32(&bar), 1);
+        tc::mbar_init(tc::smem_u32(&bar[0]), 1);
+        tc::mbar_init(tc::smem_u32(&bar[1]), 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     ncc::pdl_wait();
-    const uint32_t full = tc::smem_u32(&bar);
+    // Rows over 512 values come in two halves, the second one in flight while the first is multiplied (each half dealt to the warps).
+    const int half = (KS == kWarps && kb > 512) ? (kb / 2 + 3) & ~3 : kb;
     if (warp == 0) {
-        const uint32_t bytes = (uint32_t)kb * 4u;
         const int rows_a = (M - m0) < MT ? (M - m0) : MT, rows_b = (N - (n - lane)) < 32 ? (N - (n - lane)) : 32;
-        if (lane == 0) tc::mbar_expect_tx(full, bytes * (uint32_t)(rows_a + rows_b));
-        __syncwarp();
-        if (lane < rows_b) tc::bulk_copy(tc::smem_u32(ws + lane * wpitch), b + (long long)n * ldb + k0, bytes, full);
-        if (lane < rows_a) tc::bulk_copy(tc::smem_u32(xs + lane * chunk), a + (long long)(m0 + lane) * lda + k0, bytes, full);
+        for (int h = 0; h * half < kb; h++) {
+            const uint32_t full = tc::smem_u32(&bar[h]), bytes = (uint32_t)((kb - h * half) < half ? (kb - h * half) : half) * 4u;
+            if (lane == 0) tc::mbar_expect_tx(full, bytes * (uint32_t)(rows_a + rows_b));
+            __syncwarp();
+            if (lane < rows_b) tc::bulk_copy(tc::smem_u32(ws + lane * wpitch + h * half), b + (long long)n * ldb + k0 + h * half, bytes, full);
+            if (lane < rows_a) tc::bulk_copy(tc::smem_u32(xs + lane * chunk + h * half), a + (long long)(m0 + lane) * lda + k0 + h * half, bytes, full);
+        }
     }
     float acc[MR];
 #pragma unroll
     for (int m = 0; m < MR; m++) acc[m] = 0.f;
-    if (tc::mbar_wait(full, 0u, err, 0xD00u, &abort_flag)) {
-        const float4* wq = reinterpret_cast<const float4*>(ws + lane * wpitch + ks * slice);
-        const float4* xq = reinterpret_cast<const float4*>(xs + r0 * chunk + ks * slice);
+    bool ok = true;
+    for (int h = 0; h * half < kb && ok; h++) {
+        ok = tc::mbar_wait(tc::smem_u32(&bar[h]), 0u, err, 0xD00u + h, &abort_flag);
+        if (!ok) break;
+        // this warp's part of the half
+        const int hn = (kb - h * half) < half ? (kb - h * half) : half, part = half == kb ? slice : ((hn + KS - 1) / KS + 3) & ~3;
+        const int kn = (hn - ks * part) < part ? (hn - ks * part) : part;   // may be <= 0
+        const float4* wq = reinterpret_cast<const float4*>(ws + lane * wpitch + h * half + ks * part);
+        const float4* xq = reinterpret_cast<const float4*>(xs + r0 * chunk + h * half + ks * part);
 #pragma unroll 4
         for (int q = 0; q < kn >> 2; q++) {
             float4 w = wq[q];
@@ -76,7 +85,8 @@ __global__ void __launch_bounds__(kWarps * 32) rows_kernel(float* __restrict__ d
                 acc[m] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc[m]))));
             }
         }
-    } else {
+    }
+    if (!ok) {
         const unsigned long long t0 = tc::global_ns();   // copies in flight land before the block gives its memory back
         while (tc::global_ns() - t0 < 2000000ull) { }
     }
@@ -163,7 +173,73 @@ __global__ void __launch_bounds__(kWarps * 32) rows_odd_kernel(float* __restrict
 
 // Eight output rows x 128 columns per block; the eight warps take every eighth k and are combined in order.  a(r, k) goes through
 // shared memory as [k][8] so that one k costs a lane two broadcast reads, one 16-byte read of b and 32 multiply-adds.
-constexpr int kRT = 8, kKC = 128;
+// Up to 16 k (the input gradient of a classifier's last layer): every warp takes all of k for eight rows of its own, nothing is
+// exchanged (128 x 8192 outputs, K = 10, with its weight gradient: 22 -> 13 us).
+constexpr int kRT = 8, kKC = 128, kShortK = 16;
+
+template <bool VEC>
+__device__ __forceinline__ void columns_load(float (&bv)[4], const float* __restrict__ bp, const int (&col)[4], int C, int round_b) {
+    if (VEC) {
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (col[0] < C) q = __ldg(reinterpret_cast<const float4*>(bp + col[0]));
+        bv[0] = q.x; bv[1] = q.y; bv[2] = q.z; bv[3] = q.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) bv[e] = col[e] < C ? __ldg(bp + col[e]) : 0.f;
+    }
+    if (round_b)
+#pragma unroll
+        for (int e = 0; e < 4; e++) bv[e] = round_tf32(bv[e]);
+}
+
+template <bool VEC>
+__device__ __forceinline__ void columns_short(const ColumnsJob& j, int block, float* as) {
+    constexpr int kRows = kWarps * kRT;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = (block / j.col_tiles) * kRows, ct = block % j.col_tiles, c0 = ct * 128;
+    for (int i = threadIdx.x; i < j.K * kRows; i += kWarps * 32) {
+        const int kk = j.a_sk == 1 ? i % j.K : i / kRows, r = j.a_sk == 1 ? i / j.K : i % kRows;
+        as[kk * kRows + r] = r0 + r < j.R ? j.a[(long long)(r0 + r) * j.a_sr + (long long)kk * j.a_sk] : 0.f;
+    }
+    __syncthreads();
+    int col[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) col[e] = VEC ? c0 + lane * 4 + e : c0 + lane + 32 * e;
+    float acc[kRT][4];
+#pragma unroll
+    for (int r = 0; r < kRT; r++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[r][e] = 0.f;
+#pragma unroll 4
+    for (int kk = 0; kk < j.K; kk++) {
+        float bv[4];
+        columns_load<VEC>(bv, j.b + (long long)kk * j.ldb, col, j.C, j.round_b);
+#pragma unroll
+        for (int r = 0; r < kRT; r++) {
+            const float av = as[kk * kRows + warp * kRT + r];
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[r][e] = fmaf(av, bv[e], acc[r][e]);
+        }
+    }
+    const bool vec_out = VEC && j.ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(j.d) & 15u) == 0;
+#pragma unroll
+    for (int r = 0; r < kRT; r++) {
+        const int row = r0 + warp * kRT + r;
+        if (row >= j.R) break;
+        float* d = j.d + (long long)row * j.ldd;
+        if (vec_out) {
+            if (col[0] < j.C) *reinterpret_cast<float4*>(d + col[0]) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++) if (col[e] < j.C) d[col[e]] = acc[r][e];
+        }
+    }
+    if (j.row_sums && ct == 0 && threadIdx.x < kRows && r0 + (int)threadIdx.x < j.R) {
+        double s = 0.0;
+        for (int kk = 0; kk < j.K; kk++) s += (double)as[kk * kRows + threadIdx.x];
+        j.row_sums[r0 + threadIdx.x] = (float)s;
+    }
+}
 
 template <bool VEC>
 __device__ __forceinline__ void columns_job(const ColumnsJob& j, int block, float* as, float* red) {
@@ -192,19 +268,8 @@ __device__ __forceinline__ void columns_job(const ColumnsJob& j, int block, floa
             for (int kk = lane; kk < kn; kk += 32) rowsum += (double)as[kk * kRT + warp];
 #pragma unroll 4
         for (int kk = warp; kk < kn; kk += kWarps) {
-            const float* bp = j.b + (long long)(k0 + kk) * j.ldb;
             float bv[4];
-            if (VEC) {
-                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (col[0] < j.C) q = __ldg(reinterpret_cast<const float4*>(bp + col[0]));
-                bv[0] = q.x; bv[1] = q.y; bv[2] = q.z; bv[3] = q.w;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; e++) bv[e] = col[e] < j.C ? __ldg(bp + col[e]) : 0.f;
-            }
-            if (j.round_b)
-#pragma unroll
-                for (int e = 0; e < 4; e++) bv[e] = round_tf32(bv[e]);
+            columns_load<VEC>(bv, j.b + (long long)(k0 + kk) * j.ldb, col, j.C, j.round_b);
             const float4 a0 = *reinterpret_cast<const float4*>(as + kk * kRT), a1 = *reinterpret_cast<const float4*>(as + kk * kRT + 4);
             const float av[kRT] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
@@ -241,7 +306,10 @@ __global__ void __launch_bounds__(kWarps * 32) columns_kernel(ColumnsJob j0, Col
     const bool second = (int)blockIdx.x >= j0.blocks;
     const ColumnsJob& j = second ? j1 : j0;
     const int block = second ? (int)blockIdx.x - j0.blocks : (int)blockIdx.x;
-    if (j.vec) columns_job<true>(j, block, as, red);
+    if (j.K <= kShortK) {
+        if (j.vec) columns_short<true>(j, block, as);
+        else columns_short<false>(j, block, as);
+    } else if (j.vec) columns_job<true>(j, block, as, red);
     else columns_job<false>(j, block, as, red);
 }
 
@@ -291,7 +359,8 @@ int small_rows(float* d, long long ldd, const float* a, long long lda, const flo
 
 static void finish_job(ColumnsJob& j) {
     j.col_tiles = (j.C + 127) / 128;
-    j.blocks = j.d ? (int)((long long)((j.R + kRT - 1) / kRT) * j.col_tiles) : 0;
+    const int rows = j.K <= kShortK ? kWarps * kRT : kRT;
+    j.blocks = j.d ? (int)((long long)((j.R + rows - 1) / rows) * j.col_tiles) : 0;
     j.vec = j.C % 4 == 0 && j.ldb % 4 == 0 && al16(j.b);
 }
 int small_columns(ColumnsJob j0, ColumnsJob j1, cudaStream_t st) {
