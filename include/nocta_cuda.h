@@ -16,8 +16,9 @@
  *   - Activations are f32; 4-D tensors are NCHW for the legacy names and NHWC (channels-last)
  *     for the *_nhwc names used by the host library's own device layout.
  *   - Contractions run on tcgen05 tensor cores in TF32 (math mode 0), TF32 with
- *     round-to-nearest operand conditioning (mode 1) or 3xTF32 (mode 2) when the shape can be
- *     tiled for TMA, otherwise on an FP32 SIMT kernel; see nc_cuda_set_math_mode.
+ *     round-to-nearest operand conditioning (mode 1) or 3xTF32 (mode 2) from a certain size on
+ *     (convolutions of 16 and more channels with stride 1 or 2, products of 2^22 multiply-adds),
+ *     otherwise on FP32 CUDA-core kernels; FP32 everywhere is mode 3 (nc_cuda_set_math_mode).
  */
 #ifndef NOCTA_CUDA_ABI_H
 #define NOCTA_CUDA_ABI_H
